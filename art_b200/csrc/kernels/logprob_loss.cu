@@ -9,9 +9,11 @@
 // with the per-token weight already folded with mask / normaliser, accumulating the
 // loss terms and emitting dLoss/dlogprob for the backward pass.
 //
-// Backward recomputes the logit tiles with the same pipeline and writes
+// The gradient is
 //     dlogit[t, v] = coef[t] * (onehot(target_t)[v] - exp(logit[t, v] - lse[t]))
-// as bf16; a plain TN GEMM against the resident transposed LM head then gives dH.
+// as bf16; a plain TN GEMM against the resident transposed LM head then gives dH.  A training step lets the forward
+// write its logits in fp32 for a bounded number of rows and turns them into dlogits in place (dlogits_inplace_kernel);
+// a caller that kept no logits recomputes the tiles with the same pipeline (EpiDLogits).
 // In a vocab-parallel (TP) layout each rank runs this over its vocabulary shard and
 // the 3-float partials are what ranks exchange.
 //
@@ -53,7 +55,8 @@ struct SchedVocabSplit {
 struct EpiStats {
   const int* target;   // [M] target vocabulary id per row (global id, minus vocab_offset locally)
   float* partials;     // [splits, M, 4]  (max, sumexp, z_target, unused)
-  int M, V, vocab_offset;
+  float* logits;       // [M, ldl] fp32, or null: not kept
+  int M, V, ldl, vocab_offset;
   float run_max, run_sum, z;
   int tgt;
 
@@ -69,6 +72,13 @@ struct EpiStats {
   __device__ void chunk(const TileInfo& ti, int row, int c, uint32_t (&acc)[32]) {
     const int gc = ti.n_blk * LP_BN + c;
     if (gc >= V) return;
+    const int gr = ti.m_blk * GEMM_BM + row;
+    if (logits && gr < M) {
+      float* o = logits + static_cast<size_t>(gr) * ldl + gc;
+#pragma unroll
+      for (int j = 0; j < 32; j += 4)
+        if (gc + j < ldl) *reinterpret_cast<uint4*>(o + j) = make_uint4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+    }
     float cmax = -INFINITY;
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
@@ -323,6 +333,50 @@ __global__ void grpo_token_kernel(const float* __restrict__ partials, int splits
   }
 }
 
+// Logits -> dlogits in place: row t of `buf` holds its V fp32 logits on entry and, from the row's start, ldl bf16 gradients on
+// exit (columns V..ldl-1 zero), so the product behind it reads rows of 2 * ldl bf16.  One block per row.  A step loads
+// DL_STEP logits, and only when all threads hold theirs does any of them store: the stores of step c end at byte
+// 2 (c + 1) DL_STEP, behind every load of step c and below every load of step c + 1 (byte 4 (c + 1) DL_STEP on).
+// Bound by HBM: 4 bytes read and 2 written per logit; 1734 rows x 152 064 in 242 us = 6.5 TB/s, where recomputing the tiles
+// took 1746 us (K = 3584) and 492 us (K = 896).
+constexpr int DL_THREADS = 512;
+constexpr int DL_STEP = DL_THREADS * 8;
+
+__global__ void __launch_bounds__(DL_THREADS)
+dlogits_inplace_kernel(float* buf, int ldl, const int* __restrict__ target, const float* __restrict__ lse,
+                       const float* __restrict__ coef, int V, int vocab_offset) {
+  const int t = blockIdx.x;
+  float* row = buf + static_cast<size_t>(t) * ldl;
+  __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(row);
+  const float l = lse[t], k = coef[t];
+  const int tgt = target[t] - vocab_offset;
+  float4 a[2];
+  auto load = [&](int v) {
+    a[0] = a[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (v < V) {                         // ldl is a multiple of 8: the 8 floats are in the row
+      a[0] = *reinterpret_cast<const float4*>(row + v);
+      a[1] = *reinterpret_cast<const float4*>(row + v + 4);
+    }
+  };
+  int v = threadIdx.x * 8;
+  load(v);
+  for (int c0 = 0; c0 < ldl; c0 += DL_STEP, v += DL_STEP) {
+    const float z[8] = {a[0].x, a[0].y, a[0].z, a[0].w, a[1].x, a[1].y, a[1].z, a[1].w};
+    uint32_t packed[4];
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      float d0 = k * ((v + j == tgt ? 1.f : 0.f) - __expf(z[j] - l));
+      float d1 = k * ((v + j + 1 == tgt ? 1.f : 0.f) - __expf(z[j + 1] - l));
+      if (v + j >= V) d0 = 0.f;
+      if (v + j + 1 >= V) d1 = 0.f;
+      packed[j >> 1] = pack_bf16x2(d0, d1);
+    }
+    __syncthreads();                     // every thread's logits of this step are in registers
+    load(v + DL_STEP);
+    if (v < ldl) *reinterpret_cast<uint4*>(out + v) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+  }
+}
+
 // From this many token rows on, the LM-head kernels run on CTA pairs (256 x 256 logit tiles, the pair shares each
 // LM-head tile in shared memory); below it (decode batches) one CTA per 128 x 256 tile fills the machine better.
 static bool lp_pairs(int M) { return M >= 4 * GEMM_BM; }
@@ -391,14 +445,18 @@ ARTB_EXPORT int artb_logprob_splits(int M, int V) {
   return splits;
 }
 
-// Phase 1: per-split online-softmax partials over the vocabulary shard W[V, K].
+// Phase 1: per-split online-softmax partials over the vocabulary shard W[V, K]; with `logits` ([M, ldl] fp32, ldl >= V and a
+// multiple of 8) the logits are kept for artb_dlogits_inplace.
 ARTB_EXPORT int artb_logprob_partials(const void* H, int ldh, const void* W, int ldw, const int* target,
-                                      float* partials, int M, int V, int K, int splits, int vocab_offset,
-                                      int* status, cudaStream_t stream) {
-  if (M <= 0 || V <= 0 || (K & 7)) return ERR_BAD_SHAPE;
+                                      float* partials, float* logits, int ldl, int M, int V, int K, int splits,
+                                      int vocab_offset, int* status, cudaStream_t stream) {
+  if (M <= 0 || V <= 0 || (K & 7) || (logits && (ldl < V || (ldl & 7)))) return ERR_BAD_SHAPE;
+  if (reinterpret_cast<uintptr_t>(logits) & 15) return ERR_BAD_ALIGN;
   EpiStats epi;
   epi.target = target;
   epi.partials = partials;
+  epi.logits = logits;
+  epi.ldl = ldl;
   epi.M = M;
   epi.V = V;
   epi.vocab_offset = vocab_offset;
@@ -444,6 +502,16 @@ ARTB_EXPORT int artb_logprob_dlogits(const void* H, int ldh, const void* W, int 
   // vocab-split schedule so LM-head tiles are shared through L2 the same way.
   int splits = artb_logprob_splits(M, V);
   return launch_lp(H, ldh, W, ldw, M, V, K, splits, epi, status, stream);
+}
+
+// Backward phase 1 from kept logits: buf [M, ldl] fp32 -> rows of ldl bf16 dlogits at the start of each row (see the kernel).
+ARTB_EXPORT int artb_dlogits_inplace(float* buf, int ldl, const int* target, const float* lse, const float* coef, int M, int V,
+                                     int vocab_offset, cudaStream_t stream) {
+  if (M <= 0) return 0;
+  if (V <= 0 || ldl < V || (ldl & 7)) return ERR_BAD_SHAPE;
+  if (reinterpret_cast<uintptr_t>(buf) & 15) return ERR_BAD_ALIGN;
+  dlogits_inplace_kernel<<<M, DL_THREADS, 0, stream>>>(buf, ldl, target, lse, coef, V, vocab_offset);
+  return static_cast<int>(cudaGetLastError());
 }
 
 // Rollout sampling: partials [splits, M, 8] for one vocabulary shard (see EpiSample).

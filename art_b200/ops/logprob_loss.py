@@ -18,7 +18,8 @@ vp, ci, cf = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
 _bound: dict[str, object] = {}
 _sigs = {
     "artb_logprob_splits": [ci, ci],
-    "artb_logprob_partials": [vp, ci, vp, ci, vp, vp, ci, ci, ci, ci, ci, vp, vp],
+    "artb_logprob_partials": [vp, ci, vp, ci, vp, vp, vp, ci, ci, ci, ci, ci, ci, vp, vp],
+    "artb_dlogits_inplace": [vp, ci, vp, vp, vp, ci, ci, ci, vp],
     "artb_grpo_tokens": [vp, ci, ci, vp, vp, vp, vp, cf, cf, cf, vp, vp, vp, vp, vp],
     "artb_logprob_dlogits": [vp, ci, vp, ci, vp, vp, vp, vp, ci, ci, ci, ci, ci, vp, vp],
 }
@@ -42,15 +43,17 @@ class LogprobResult:
     accum: torch.Tensor | None  # [4] fp32: sum(pg*w), sum(kl*w), #tokens with w != 0
 
 
-def partials(hidden: torch.Tensor, lm_head: torch.Tensor, target: torch.Tensor, vocab_offset: int = 0
-             ) -> tuple[torch.Tensor, int]:
-    """Per-vocab-split (max, sumexp, z_target) for one vocabulary shard: [splits, M, 4] fp32."""
+def partials(hidden: torch.Tensor, lm_head: torch.Tensor, target: torch.Tensor, vocab_offset: int = 0,
+             logits: torch.Tensor | None = None) -> tuple[torch.Tensor, int]:
+    """Per-vocab-split (max, sumexp, z_target) for one vocabulary shard: [splits, M, 4] fp32.  ``logits`` ([M, ldl] fp32,
+    ``ldl`` a multiple of 8) also receives the logits."""
     M, K = hidden.shape
     V = lm_head.shape[0]
     splits = _f("artb_logprob_splits")(M, V)
     part = torch.empty((splits, M, 4), dtype=torch.float32, device=hidden.device)
     rc = _f("artb_logprob_partials")(_lib.ptr(hidden), hidden.stride(0), _lib.ptr(lm_head), lm_head.stride(0),
-                                     _lib.ptr(target), _lib.ptr(part), M, V, K, splits, vocab_offset,
+                                     _lib.ptr(target), _lib.ptr(part), _lib.ptr(logits),
+                                     logits.stride(0) if logits is not None else 0, M, V, K, splits, vocab_offset,
                                      _lib.ptr(_lib.status_word(hidden.device)), _lib.stream_ptr())
     _lib.check_rc(rc, "logprob_partials")
     return part, splits
@@ -92,6 +95,40 @@ def backward(hidden, lm_head, lm_head_t, target, lse, coef, dlogits_buf: torch.T
                                     _lib.ptr(_lib.status_word(hidden.device)), _lib.stream_ptr())
     _lib.check_rc(rc, "logprob_dlogits")
     return gemm_tn(dl, lm_head_t)
+
+
+LOGIT_ROWS = 2048     # at most this many rows' logits are alive at once, or half of the batch's (see forward_backward)
+
+
+def forward_backward(hidden, lm_head, lm_head_t, target, old_lp, adv, tok_w, ref_lp=None, eps_lo=0.2, eps_hi=0.2, beta=0.0,
+                     accum=None) -> tuple[LogprobResult, torch.Tensor]:
+    """Loss terms of the rows of ``hidden`` and dLoss/dhidden [M,K] bf16, the logits computed once.
+
+    The rows of a batch are independent, so it is cut into pieces whose fp32 logits are kept from the forward to the
+    gradient: half of the rows, which is what all rows' bf16 dlogits would take, or ``LOGIT_ROWS`` where that is more.
+    """
+    M, K = hidden.shape
+    V, ldl = lm_head.shape[0], lm_head_t.shape[1]
+    piece = max(LOGIT_ROWS, ((M + 1) // 2 + 255) // 256 * 256)
+    dh = torch.empty((M, K), dtype=torch.bfloat16, device=hidden.device)
+    buf = torch.empty((min(piece, M), ldl), dtype=torch.float32, device=hidden.device)
+    parts = []
+    for m0 in range(0, M, piece):
+        s = slice(m0, min(M, m0 + piece))
+        n = s.stop - m0
+        cut = lambda t: None if t is None else t[s]  # noqa: E731
+        part, _ = partials(hidden[s], lm_head, target[s], logits=buf)
+        res = grpo_tokens(part, cut(old_lp), cut(adv), cut(tok_w), cut(ref_lp), eps_lo, eps_hi, beta, accum)
+        accum = res.accum
+        rc = _f("artb_dlogits_inplace")(_lib.ptr(buf), ldl, _lib.ptr(target[s]), _lib.ptr(res.lse), _lib.ptr(res.coef), n, V, 0,
+                                        _lib.stream_ptr())
+        _lib.check_rc(rc, "dlogits_inplace")
+        gemm_tn(buf.view(torch.bfloat16)[:n, :ldl], lm_head_t, out=dh[s])
+        parts.append(res)
+    if len(parts) == 1:
+        return parts[0], dh
+    join = lambda k: torch.cat([getattr(r, k) for r in parts])  # noqa: E731
+    return LogprobResult(join("logprobs"), join("lse"), join("coef"), accum), dh
 
 
 def reference_logprobs(hidden, lm_head, target):

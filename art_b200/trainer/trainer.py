@@ -280,9 +280,8 @@ class Trainer:
                 ref_c = lpl.grpo_tokens(part).logprobs
                 del ref_hidden, rc, part
             with self.timer.phase("lm_head_loss"):
-                res = lpl.forward(hc, self.model.lm_head, tgt_c, old_c, adv_c, w_c, ref_c, hyper.epsilon, eps_hi,
-                                  hyper.beta, accum)
-                dhc = lpl.backward(hc, self.model.lm_head, self.model.lm_head_t, tgt_c, res.lse, res.coef)
+                _, dhc = lpl.forward_backward(hc, self.model.lm_head, self.model.lm_head_t, tgt_c, old_c, adv_c, w_c, ref_c,
+                                              hyper.epsilon, eps_hi, hyper.beta, accum)
                 dhidden = torch.zeros_like(hidden)
                 ew.scatter_rows_(dhc, sel, dhidden)
                 del hc, dhc
@@ -353,9 +352,8 @@ class Trainer:
                     adv_c = shift_left(rows_d["advantages"][r0:r1], 0.0).reshape(-1)[sel]
                     hc = ew.gather_rows(hidden, sel)
                     with trainer.timer.phase("lm_head_loss"):
-                        res = lpl.forward(hc, model.lm_head, target[sel], old_c, adv_c, w_flat[sel], ref_lp.get(mb),
-                                          hyper.epsilon, eps_hi, hyper.beta, accum)
-                        dhc = lpl.backward(hc, model.lm_head, model.lm_head_t, target[sel], res.lse, res.coef)
+                        _, dhc = lpl.forward_backward(hc, model.lm_head, model.lm_head_t, target[sel], old_c, adv_c,
+                                                      w_flat[sel], ref_lp.get(mb), hyper.epsilon, eps_hi, hyper.beta, accum)
                     ew.scatter_rows_(dhc, sel, dhidden)
                 self.live[mb] = (saved, final, dhidden)
                 return None
