@@ -34,6 +34,7 @@ import torch
 from ..ops import attention as attn_ops
 from ..ops import elementwise as ew
 from ..ops.gemm import gemm_tn, skinny_gemm
+from ..ops.lora_pack import LoraTable
 from .config import ModelConfig
 from .weights import LoraConfig, lora_key
 
@@ -331,6 +332,10 @@ class NativeDecoder:
                 layer["q_norm"] = base[p + "self_attn.q_norm.weight"].to(dev, bf).contiguous()
                 layer["k_norm"] = base[p + "self_attn.k_norm.weight"].to(dev, bf).contiguous()
             self.layers.append(layer)
+        # plain fused linears: one launch for all of them; the grouped ones of sparse layers already take few
+        linears = list(self.linears())
+        self._table = LoraTable([lin for lin in linears if isinstance(lin, LoraLinear)])
+        self._grouped = [lin for lin in linears if not isinstance(lin, LoraLinear)]
         self.refresh_lora()
 
     # -- LoRA bookkeeping -------------------------------------------------------------------
@@ -340,16 +345,19 @@ class NativeDecoder:
             yield layer["o"]
             yield from layer["mlp"].linears()
 
+    def _lora(self):
+        return (self._table, *self._grouped)
+
     def refresh_lora(self) -> None:
-        for lin in self.linears():
+        for lin in self._lora():
             lin.refresh()
 
     def zero_grad(self) -> None:
-        for lin in self.linears():
+        for lin in self._lora():
             lin.zero_grad()
 
     def export_grads(self) -> None:
-        for lin in self.linears():
+        for lin in self._lora():
             lin.export_grads()
 
     # -- forward ----------------------------------------------------------------------------
