@@ -1,16 +1,16 @@
-// Tree-masked flash attention backward on tcgen05 / TMEM (head dim 128), two kernels without atomics.
+// Tree-masked flash attention backward on tcgen05 / TMEM (head dims 64 and 128), two kernels without atomics.
 //
 //   dkv kernel  one CTA per (128-key block, kv head); items = (query head of the group, 64-query block):
-//       S^T  = K Q^T            UMMA 128 x 64 x 128   A = K tile (resident)   B = Q tile
-//       dP^T = V dO^T           UMMA 128 x 64 x 128   A = V tile (resident)   B = dO tile
+//       S^T  = K Q^T            UMMA 128 x 64 x HD    A = K tile (resident)   B = Q tile
+//       dP^T = V dO^T           UMMA 128 x 64 x HD    A = V tile (resident)   B = dO tile
 //       P^T  = exp2(S^T c - lse),  dS^T = c' P^T (dP^T - D)      thread = key row (TMEM lane), bf16 rows
 //                                                                 written to shared memory, swizzled K-major
-//       dV  += P^T dO           UMMA 128 x 128 x 64   A = P^T        B = dO^T tile (pre-transposed copy)
-//       dK  += dS^T Q           UMMA 128 x 128 x 64   A = dS^T       B = Q^T tile  (pre-transposed copy)
+//       dV  += P^T dO           UMMA 128 x HD x 64    A = P^T        B = dO^T tile (pre-transposed copy)
+//       dK  += dS^T Q           UMMA 128 x HD x 64    A = dS^T       B = Q^T tile  (pre-transposed copy)
 //     dK and dV accumulate in TMEM over every item (all query heads of the group), so GQA needs no atomics.
 //   dq kernel   one CTA per (128-query block, query head); items = 64-key blocks:
-//       S = Q K^T,  dP = dO V^T  (128 x 64 x 128),  dS = c' P (dP - D)  thread = query row,
-//       dQ += dS K               UMMA 128 x 128 x 64   A = dS   B = K^T tile (pre-transposed copy)
+//       S = Q K^T,  dP = dO V^T  (128 x 64 x HD),  dS = c' P (dP - D)  thread = query row,
+//       dQ += dS K               UMMA 128 x HD x 64    A = dS   B = K^T tile (pre-transposed copy)
 //
 // Every operand is K-major with the 128-byte swizzle (the layout TMA writes and the only one this code base
 // has validated); the three transposed copies (Q^T, dO^T, K^T: ~125 MB per layer at 8192 tokens) cost ~0.05 ms
@@ -29,7 +29,6 @@
 
 namespace artb {
 
-constexpr int TB_HD = 128;
 constexpr int TB_THREADS = 576;   // TMA warp, MMA warp, 16 element-wise warps (four per TMEM lane quarter)
 
 __device__ __forceinline__ float tb_ex2(float x) {
@@ -48,16 +47,19 @@ __device__ __forceinline__ uint64_t tb_desc_r64(uint32_t base, int kk) {
 __device__ __forceinline__ uint64_t tb_desc_c64(uint32_t base, int kk) { return umma_smem_desc_k128(base) + 2 * kk; }
 
 // ============================================================================================ dK / dV
+template <int HD>
 struct DkvSmem {
-  static constexpr int K = 0, V = 32768;
-  static constexpr int STAGE = 65536;              // [2] x { Q 16K | dO 16K | Q^T 16K | dO^T 16K }
-  static constexpr int PT = STAGE + 2 * 65536;     // P^T  [128 x 64] bf16
+  static constexpr int TILE = 128 * HD * 2, PIECE = 64 * HD * 2;
+  static constexpr int K = 0, V = TILE;
+  static constexpr int STAGE = 2 * TILE;           // [2] x { Q | dO | Q^T | dO^T }, a PIECE each
+  static constexpr int PT = STAGE + 8 * PIECE;     // P^T  [128 x 64] bf16
   static constexpr int DST = PT + 16384;           // dS^T [128 x 64] bf16
   static constexpr int LD = DST + 16384;           // float2 [16 warps][16]: (lse2, D) of the warp's 16 queries
   static constexpr int BAR = LD + 4 * 64 * 8;
-  static constexpr int TOTAL = BAR + 256;          // 231 680 B; the dynamic window must start 1024-aligned
+  static constexpr int TOTAL = BAR + 256;          // 231 680 B at 128; the dynamic window must start 1024-aligned
 };
 
+template <int HD>
 __global__ void __launch_bounds__(TB_THREADS, 1)
 attn_tc_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV128, const __grid_constant__ CUtensorMap tmQKV64,
                    const __grid_constant__ CUtensorMap tmDO64, const __grid_constant__ CUtensorMap tmQt,
@@ -65,8 +67,10 @@ attn_tc_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV128, const __grid_co
                    const uint8_t* __restrict__ state, const float* __restrict__ lse2, const float* __restrict__ Dv,
                    __nv_bfloat16* __restrict__ dqkv, int ld, int S, int Hq, int Hkv, float scale, float scale_log2, long M,
                    int GS, float* __restrict__ partial, int* status) {
+  using L = DkvSmem<HD>;
+  constexpr int P = L::PIECE;
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + DkvSmem::BAR);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR);
   uint64_t* kv_full = bars;
   uint64_t* stage_full = bars + 1;    // [2]
   uint64_t* stage_empty = bars + 3;   // [2]
@@ -129,11 +133,12 @@ attn_tc_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV128, const __grid_co
   if (warp == 0) {
     if (lane == 0) {
       const int krow = static_cast<int>(base) + kb * 128;
-      mbar_expect_tx(kv_full, 65536);
-      tma_load_2d(smem + DkvSmem::K, &tmQKV128, (Hq + kvh) * TB_HD, krow, kv_full);
-      tma_load_2d(smem + DkvSmem::K + 16384, &tmQKV128, (Hq + kvh) * TB_HD + 64, krow, kv_full);
-      tma_load_2d(smem + DkvSmem::V, &tmQKV128, (Hq + Hkv + kvh) * TB_HD, krow, kv_full);
-      tma_load_2d(smem + DkvSmem::V + 16384, &tmQKV128, (Hq + Hkv + kvh) * TB_HD + 64, krow, kv_full);
+      mbar_expect_tx(kv_full, 2 * L::TILE);
+#pragma unroll
+      for (int c = 0; c < HD; c += 64) {
+        tma_load_2d(smem + L::K + c * 256, &tmQKV128, (Hq + kvh) * HD + c, krow, kv_full);
+        tma_load_2d(smem + L::V + c * 256, &tmQKV128, (Hq + Hkv + kvh) * HD + c, krow, kv_full);
+      }
       uint32_t it = 0;
       for (int item = 0; item < n_items && !*abort_flag; ++item) {
         int g, qb;
@@ -146,34 +151,35 @@ attn_tc_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV128, const __grid_co
         }
         const int hq = kvh * Gall + g_lo + g;
         const int qrow = static_cast<int>(base) + qb * 64;
-        uint8_t* st = smem + DkvSmem::STAGE + s * 65536;
-        mbar_expect_tx(&stage_full[s], 65536);
-        tma_load_2d(st, &tmQKV64, hq * TB_HD, qrow, &stage_full[s]);
-        tma_load_2d(st + 8192, &tmQKV64, hq * TB_HD + 64, qrow, &stage_full[s]);
-        tma_load_2d(st + 16384, &tmDO64, hq * TB_HD, qrow, &stage_full[s]);
-        tma_load_2d(st + 24576, &tmDO64, hq * TB_HD + 64, qrow, &stage_full[s]);
-        tma_load_2d(st + 32768, &tmQt, qrow, hq * TB_HD, &stage_full[s]);
-        tma_load_2d(st + 49152, &tmDOt, qrow, hq * TB_HD, &stage_full[s]);
+        uint8_t* st = smem + L::STAGE + s * 4 * P;
+        mbar_expect_tx(&stage_full[s], 4 * P);
+#pragma unroll
+        for (int c = 0; c < HD; c += 64) {
+          tma_load_2d(st + c * 128, &tmQKV64, hq * HD + c, qrow, &stage_full[s]);
+          tma_load_2d(st + P + c * 128, &tmDO64, hq * HD + c, qrow, &stage_full[s]);
+        }
+        tma_load_2d(st + 2 * P, &tmQt, qrow, hq * HD, &stage_full[s]);
+        tma_load_2d(st + 3 * P, &tmDOt, qrow, hq * HD, &stage_full[s]);
         ++it;
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      constexpr uint32_t id_s = umma_idesc_bf16(128, 64), id_acc = umma_idesc_bf16(128, 128);
-      const uint32_t sK = smem_u32(smem + DkvSmem::K), sV = smem_u32(smem + DkvSmem::V);
-      const uint32_t sPT = smem_u32(smem + DkvSmem::PT), sDST = smem_u32(smem + DkvSmem::DST);
+      constexpr uint32_t id_s = umma_idesc_bf16(128, 64), id_acc = umma_idesc_bf16(128, HD);
+      const uint32_t sK = smem_u32(smem + L::K), sV = smem_u32(smem + L::V);
+      const uint32_t sPT = smem_u32(smem + L::PT), sDST = smem_u32(smem + L::DST);
       bool ok = mbar_wait(kv_full, 0);
       auto issue_acc = [&](uint32_t i) -> bool {
         const int s = i & 1;
         if (!mbar_wait(pt_full, i & 1)) return false;
         tc_fence_after_sync();
-        const uint32_t st = smem_u32(smem + DkvSmem::STAGE + s * 65536);
+        const uint32_t st = smem_u32(smem + L::STAGE + s * 4 * P);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-          tc_mma_f16(tmem + 256, tb_desc_c64(sPT, kk), tb_desc_c64(st + 49152, kk), id_acc, (i | kk) != 0);
+          tc_mma_f16(tmem + 256, tb_desc_c64(sPT, kk), tb_desc_c64(st + 3 * P, kk), id_acc, (i | kk) != 0);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-          tc_mma_f16(tmem + 384, tb_desc_c64(sDST, kk), tb_desc_c64(st + 32768, kk), id_acc, (i | kk) != 0);
+          tc_mma_f16(tmem + 256 + HD, tb_desc_c64(sDST, kk), tb_desc_c64(st + 2 * P, kk), id_acc, (i | kk) != 0);
         tc_commit(&stage_empty[s]);
         tc_commit(pt_empty);
         return true;
@@ -189,13 +195,13 @@ attn_tc_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV128, const __grid_co
           break;
         }
         tc_fence_after_sync();
-        const uint32_t st = smem_u32(smem + DkvSmem::STAGE + s * 65536);
+        const uint32_t st = smem_u32(smem + L::STAGE + s * 4 * P);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
+        for (int kk = 0; kk < HD / 16; ++kk)
           tc_mma_f16(tmem + s * 64, tb_desc_r128(sK, kk), tb_desc_r64(st, kk), id_s, kk != 0);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          tc_mma_f16(tmem + 128 + s * 64, tb_desc_r128(sV, kk), tb_desc_r64(st + 16384, kk), id_s, kk != 0);
+        for (int kk = 0; kk < HD / 16; ++kk)
+          tc_mma_f16(tmem + 128 + s * 64, tb_desc_r128(sV, kk), tb_desc_r64(st + P, kk), id_s, kk != 0);
         tc_commit(&s_full[s]);
         if (it > 0 && !issue_acc(it - 1)) {
           ok = false;
@@ -219,9 +225,9 @@ attn_tc_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV128, const __grid_co
     const int gk_mine = gid[ki];
     const int kpos = kb * 128 + r;
     const uint32_t lane_off = static_cast<uint32_t>(q * 32) << 16;
-    float2* ldw = reinterpret_cast<float2*>(smem + DkvSmem::LD) + (q * 4 + hf) * 16;   // (lse2, D) of my 16 queries
-    uint8_t* pt_row = smem + DkvSmem::PT + r * 128;
-    uint8_t* dst_row = smem + DkvSmem::DST + r * 128;
+    float2* ldw = reinterpret_cast<float2*>(smem + L::LD) + (q * 4 + hf) * 16;   // (lse2, D) of my 16 queries
+    uint8_t* pt_row = smem + L::PT + r * 128;
+    uint8_t* dst_row = smem + L::DST + r * 128;
     const int sw = r & 7;
     const int l16 = lane & 15;
     bool dead = false;
@@ -351,34 +357,35 @@ attn_tc_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV128, const __grid_co
     }
     if (!dead) {
       tc_fence_after_sync();
-      __nv_bfloat16* dk = dqkv + ki * ld + (Hq + kvh) * TB_HD + hf * 32;
-      __nv_bfloat16* dv = dqkv + ki * ld + (Hq + Hkv + kvh) * TB_HD + hf * 32;
-      // partial layout: fp32 [GS][M][2 * Hkv * 128], columns = dk of all kv heads, then dv of all kv heads
-      float* pk = partial ? partial + (static_cast<size_t>(gs) * M + ki) * (2 * Hkv * TB_HD) + kvh * TB_HD + hf * 32 : nullptr;
-      float* pv = partial ? pk + Hkv * TB_HD : nullptr;
+      constexpr int CW = HD / 4;     // my columns of each accumulator
+      __nv_bfloat16* dk = dqkv + ki * ld + (Hq + kvh) * HD + hf * CW;
+      __nv_bfloat16* dv = dqkv + ki * ld + (Hq + Hkv + kvh) * HD + hf * CW;
+      // partial layout: fp32 [GS][M][2 * Hkv * HD], columns = dk of all kv heads, then dv of all kv heads
+      float* pk = partial ? partial + (static_cast<size_t>(gs) * M + ki) * (2 * Hkv * HD) + kvh * HD + hf * CW : nullptr;
+      float* pv = partial ? pk + Hkv * HD : nullptr;
 #pragma unroll 1
       for (int which = 0; which < 2; ++which) {
         __nv_bfloat16* o = which == 0 ? dv : dk;
         float* po = which == 0 ? pv : pk;
         const float f = which == 0 ? 1.f : scale;
-        const uint32_t col0 = 256 + which * 128 + hf * 32;
+        const uint32_t col0 = 256 + which * HD + hf * CW;
 #pragma unroll 1
-        for (int c = 0; c < 32; c += 32) {
-          uint32_t v[32];
+        for (int c = 0; c < CW; c += 16) {
+          uint32_t v[16];
           if (it > 0) {
-            tmem_ld_32x32(tmem + lane_off + col0 + c, v);
+            tmem_ld_32x16(tmem + lane_off + col0 + c, v);
             tmem_ld_wait();
           } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = 0u;
+            for (int j = 0; j < 16; ++j) v[j] = 0u;
           }
           if (po) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(po + c + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+            for (int j = 0; j < 16; j += 4) *reinterpret_cast<uint4*>(po + c + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
             continue;
           }
 #pragma unroll
-          for (int j = 0; j < 32; j += 8) {
+          for (int j = 0; j < 16; j += 8) {
             uint4 w;
             w.x = pack_bf16x2(__uint_as_float(v[j]) * f, __uint_as_float(v[j + 1]) * f);
             w.y = pack_bf16x2(__uint_as_float(v[j + 2]) * f, __uint_as_float(v[j + 3]) * f);
@@ -404,23 +411,28 @@ attn_tc_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV128, const __grid_co
 }
 
 // ================================================================================================= dQ
+template <int HD>
 struct DqSmem {
-  static constexpr int Q = 0, DO = 32768;
-  static constexpr int STAGE = 65536;              // [2] x { K 16K | V 16K | K^T 16K }
-  static constexpr int DS = STAGE + 2 * 49152;     // [2] x dS [128 x 64] bf16
+  static constexpr int TILE = 128 * HD * 2, PIECE = 64 * HD * 2;
+  static constexpr int Q = 0, DO = TILE;
+  static constexpr int STAGE = 2 * TILE;           // [2] x { K | V | K^T }, a PIECE each
+  static constexpr int DS = STAGE + 6 * PIECE;     // [2] x dS [128 x 64] bf16
   static constexpr int GK = DS + 2 * 16384;        // int [16 warps][16]
   static constexpr int BAR = GK + 4 * 64 * 4;
   static constexpr int TOTAL = BAR + 256;
 };
 
+template <int HD>
 __global__ void __launch_bounds__(TB_THREADS, 1)
 attn_tc_dq_kernel(const __grid_constant__ CUtensorMap tmQKV128, const __grid_constant__ CUtensorMap tmQKV64,
                   const __grid_constant__ CUtensorMap tmDO128, const __grid_constant__ CUtensorMap tmKt,
                   const int* __restrict__ gid, const int* __restrict__ pid, const uint8_t* __restrict__ state,
                   const float* __restrict__ lse2, const float* __restrict__ Dv, __nv_bfloat16* __restrict__ dqkv, int ld,
                   int S, int Hq, int Hkv, float scale, float scale_log2, long M, int* status) {
+  using L = DqSmem<HD>;
+  constexpr int P = L::PIECE;
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + DqSmem::BAR);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR);
   uint64_t* qdo_full = bars;
   uint64_t* stage_full = bars + 1;    // [2]
   uint64_t* stage_empty = bars + 3;   // [2]
@@ -474,11 +486,12 @@ attn_tc_dq_kernel(const __grid_constant__ CUtensorMap tmQKV128, const __grid_con
   if (warp == 0) {
     if (lane == 0) {
       const int qrow = static_cast<int>(base) + qb * 128;
-      mbar_expect_tx(qdo_full, 65536);
-      tma_load_2d(smem + DqSmem::Q, &tmQKV128, h * TB_HD, qrow, qdo_full);
-      tma_load_2d(smem + DqSmem::Q + 16384, &tmQKV128, h * TB_HD + 64, qrow, qdo_full);
-      tma_load_2d(smem + DqSmem::DO, &tmDO128, h * TB_HD, qrow, qdo_full);
-      tma_load_2d(smem + DqSmem::DO + 16384, &tmDO128, h * TB_HD + 64, qrow, qdo_full);
+      mbar_expect_tx(qdo_full, 2 * L::TILE);
+#pragma unroll
+      for (int c = 0; c < HD; c += 64) {
+        tma_load_2d(smem + L::Q + c * 256, &tmQKV128, h * HD + c, qrow, qdo_full);
+        tma_load_2d(smem + L::DO + c * 256, &tmDO128, h * HD + c, qrow, qdo_full);
+      }
       uint32_t it = 0;
       for (int kb = 0; kb < n_items && !*abort_flag; ++kb) {
         if (item_state(kb) == 0) continue;
@@ -489,30 +502,31 @@ attn_tc_dq_kernel(const __grid_constant__ CUtensorMap tmQKV128, const __grid_con
           break;
         }
         const int krow = static_cast<int>(base) + kb * 64;
-        uint8_t* st = smem + DqSmem::STAGE + s * 49152;
-        mbar_expect_tx(&stage_full[s], 49152);
-        tma_load_2d(st, &tmQKV64, (Hq + kvh) * TB_HD, krow, &stage_full[s]);
-        tma_load_2d(st + 8192, &tmQKV64, (Hq + kvh) * TB_HD + 64, krow, &stage_full[s]);
-        tma_load_2d(st + 16384, &tmQKV64, (Hq + Hkv + kvh) * TB_HD, krow, &stage_full[s]);
-        tma_load_2d(st + 24576, &tmQKV64, (Hq + Hkv + kvh) * TB_HD + 64, krow, &stage_full[s]);
-        tma_load_2d(st + 32768, &tmKt, krow, kvh * TB_HD, &stage_full[s]);
+        uint8_t* st = smem + L::STAGE + s * 3 * P;
+        mbar_expect_tx(&stage_full[s], 3 * P);
+#pragma unroll
+        for (int c = 0; c < HD; c += 64) {
+          tma_load_2d(st + c * 128, &tmQKV64, (Hq + kvh) * HD + c, krow, &stage_full[s]);
+          tma_load_2d(st + P + c * 128, &tmQKV64, (Hq + Hkv + kvh) * HD + c, krow, &stage_full[s]);
+        }
+        tma_load_2d(st + 2 * P, &tmKt, krow, kvh * HD, &stage_full[s]);
         ++it;
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      constexpr uint32_t id_s = umma_idesc_bf16(128, 64), id_acc = umma_idesc_bf16(128, 128);
-      const uint32_t sQ = smem_u32(smem + DqSmem::Q), sDO = smem_u32(smem + DqSmem::DO);
+      constexpr uint32_t id_s = umma_idesc_bf16(128, 64), id_acc = umma_idesc_bf16(128, HD);
+      const uint32_t sQ = smem_u32(smem + L::Q), sDO = smem_u32(smem + L::DO);
       bool ok = mbar_wait(qdo_full, 0);
       auto issue_acc = [&](uint32_t i) -> bool {
         const int s = i & 1;
         if (!mbar_wait(&ds_full[s], (i >> 1) & 1)) return false;
         tc_fence_after_sync();
-        const uint32_t st = smem_u32(smem + DqSmem::STAGE + s * 49152);
-        const uint32_t sds = smem_u32(smem + DqSmem::DS + s * 16384);
+        const uint32_t st = smem_u32(smem + L::STAGE + s * 3 * P);
+        const uint32_t sds = smem_u32(smem + L::DS + s * 16384);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-          tc_mma_f16(tmem + 256, tb_desc_c64(sds, kk), tb_desc_c64(st + 32768, kk), id_acc, (i | kk) != 0);
+          tc_mma_f16(tmem + 256, tb_desc_c64(sds, kk), tb_desc_c64(st + 2 * P, kk), id_acc, (i | kk) != 0);
         tc_commit(&stage_empty[s]);
         tc_commit(&ds_empty[s]);
         return true;
@@ -527,13 +541,13 @@ attn_tc_dq_kernel(const __grid_constant__ CUtensorMap tmQKV128, const __grid_con
           break;
         }
         tc_fence_after_sync();
-        const uint32_t st = smem_u32(smem + DqSmem::STAGE + s * 49152);
+        const uint32_t st = smem_u32(smem + L::STAGE + s * 3 * P);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
+        for (int kk = 0; kk < HD / 16; ++kk)
           tc_mma_f16(tmem + s * 64, tb_desc_r128(sQ, kk), tb_desc_r64(st, kk), id_s, kk != 0);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          tc_mma_f16(tmem + 128 + s * 64, tb_desc_r128(sDO, kk), tb_desc_r64(st + 16384, kk), id_s, kk != 0);
+        for (int kk = 0; kk < HD / 16; ++kk)
+          tc_mma_f16(tmem + 128 + s * 64, tb_desc_r128(sDO, kk), tb_desc_r64(st + P, kk), id_s, kk != 0);
         tc_commit(&s_full[s]);
         if (it > 0 && !issue_acc(it - 1)) {
           ok = false;
@@ -557,7 +571,7 @@ attn_tc_dq_kernel(const __grid_constant__ CUtensorMap tmQKV128, const __grid_con
     const int qpos = qb * 128 + r;
     const float lse_r = lse2[static_cast<long>(h) * M + qi], D_r = Dv[static_cast<long>(h) * M + qi];
     const uint32_t lane_off = static_cast<uint32_t>(q * 32) << 16;
-    int* gk = reinterpret_cast<int*>(smem + DqSmem::GK) + (q * 4 + hf) * 16;
+    int* gk = reinterpret_cast<int*>(smem + L::GK) + (q * 4 + hf) * 16;
     const int sw = r & 7;
     bool dead = false;
     uint32_t it = 0;
@@ -602,7 +616,7 @@ attn_tc_dq_kernel(const __grid_constant__ CUtensorMap tmQKV128, const __grid_con
         dead = true;
         break;
       }
-      uint8_t* ds_row = smem + DqSmem::DS + s * 16384 + r * 128;
+      uint8_t* ds_row = smem + L::DS + s * 16384 + r * 128;
       const int k0 = kb * 64 + hf * 16;
 #pragma unroll
       for (int ii = 0; ii < 2; ++ii) {
@@ -641,19 +655,20 @@ attn_tc_dq_kernel(const __grid_constant__ CUtensorMap tmQKV128, const __grid_con
     }
     if (!dead) {
       tc_fence_after_sync();
-      __nv_bfloat16* o = dqkv + qi * ld + h * TB_HD + hf * 32;
+      constexpr int CW = HD / 4;
+      __nv_bfloat16* o = dqkv + qi * ld + h * HD + hf * CW;
 #pragma unroll 1
-      for (int c = 0; c < 32; c += 32) {
-        uint32_t v[32];
+      for (int c = 0; c < CW; c += 16) {
+        uint32_t v[16];
         if (it > 0) {
-          tmem_ld_32x32(tmem + lane_off + 256 + hf * 32 + c, v);
+          tmem_ld_32x16(tmem + lane_off + 256 + hf * CW + c, v);
           tmem_ld_wait();
         } else {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = 0u;
+          for (int j = 0; j < 16; ++j) v[j] = 0u;
         }
 #pragma unroll
-        for (int j = 0; j < 32; j += 8) {
+        for (int j = 0; j < 16; j += 8) {
           uint4 w;
           w.x = pack_bf16x2(__uint_as_float(v[j]) * scale, __uint_as_float(v[j + 1]) * scale);
           w.y = pack_bf16x2(__uint_as_float(v[j + 2]) * scale, __uint_as_float(v[j + 3]) * scale);
@@ -732,89 +747,121 @@ attn_tc_transpose_kernel(const __nv_bfloat16* __restrict__ src, int ld, int c0, 
   }
 }
 
-// D[h, m] = sum_d dO[m, h*128 + d] * O[m, h*128 + d]   (one warp per (token, head))
+// D[h, m] = sum_d dO[m, h*HD + d] * O[m, h*HD + d]   (one warp per 128 columns of a token: one or two heads)
+template <int HD>
 __global__ void attn_tc_rowdot_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O, int ld,
                                       float* __restrict__ D, long M, int Hq) {
+  constexpr int LANES = HD / 4;      // lanes per head
+  const int per_token = (Hq * HD + 127) / 128;
   const long wid = blockIdx.x * static_cast<long>(blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (wid >= M * Hq) return;
-  const long m = wid / Hq;
-  const int h = static_cast<int>(wid % Hq);
-  const uint2 a = *reinterpret_cast<const uint2*>(dO + m * ld + h * TB_HD + lane * 4);
-  const uint2 b = *reinterpret_cast<const uint2*>(O + m * ld + h * TB_HD + lane * 4);
-  const float2 a0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a.x));
-  const float2 a1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a.y));
-  const float2 b0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&b.x));
-  const float2 b1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&b.y));
-  float s = a0.x * b0.x + a0.y * b0.y + a1.x * b1.x + a1.y * b1.y;
+  if (wid >= M * per_token) return;
+  const long m = wid / per_token;
+  const int h = static_cast<int>(wid % per_token) * (32 / LANES) + lane / LANES;
+  float s = 0.f;
+  if (h < Hq) {
+    const long at = m * ld + h * HD + (lane % LANES) * 4;
+    const uint2 a = *reinterpret_cast<const uint2*>(dO + at);
+    const uint2 b = *reinterpret_cast<const uint2*>(O + at);
+    const float2 a0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a.x));
+    const float2 a1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a.y));
+    const float2 b0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&b.x));
+    const float2 b1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&b.y));
+    s = a0.x * b0.x + a0.y * b0.y + a1.x * b1.x + a1.y * b1.y;
+  }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) D[static_cast<long>(h) * M + m] = s;
+  for (int o = LANES / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane % LANES == 0 && h < Hq) D[static_cast<long>(h) * M + m] = s;
 }
 
 }  // namespace artb
 
 using namespace artb;
 
-// qkv / dqkv [rows*S, ld] (q | k | v columns); out, dout [rows*S, ldo]; lse2, Dbuf fp32 [Hq, rows*S];
-// scratch bf16: qt, dot [Hq*128, rows*S], kt [Hkv*128, rows*S]; partial: optional fp32 [2, rows*S, 2*Hkv*128]
-// (enables the two-way split of a kv group's query heads).  Head dim 128, S % 128 == 0.
-ARTB_EXPORT int artb_attn_tc_bwd(const void* qkv, int ld, const void* out, const void* dout, int ldo, const int* gid,
-                                 const int* pid, const uint8_t* state, const float* lse2, float* Dbuf, void* qt, void* dot,
-                                 void* kt, void* dqkv, float* partial, int rows, int S, int Hq, int Hkv, int* status,
-                                 cudaStream_t st) {
-  if (S % 128 || Hq % Hkv || (ld & 7) || (ldo & 7)) return ERR_BAD_SHAPE;
+namespace artb {
+
+template <int HD>
+static int launch_tc_bwd(const void* qkv, int ld, const void* out, const void* dout, int ldo, const int* gid, const int* pid,
+                         const uint8_t* state, const float* lse2, float* Dbuf, void* qt, void* dot, void* kt, void* dqkv,
+                         float* partial, int GS, int rows, int S, int Hq, int Hkv, int* status, cudaStream_t st) {
   const long M = static_cast<long>(rows) * S;
-  if (M > 0x7fffffffL) return ERR_BAD_SHAPE;
   typedef __nv_bfloat16 bf;
   {
-    const long warps = M * Hq;
-    attn_tc_rowdot_kernel<<<static_cast<unsigned>((warps + 3) / 4), 128, 0, st>>>(
+    const long warps = M * ((Hq * HD + 127) / 128);
+    attn_tc_rowdot_kernel<HD><<<static_cast<unsigned>((warps + 3) / 4), 128, 0, st>>>(
         reinterpret_cast<const bf*>(dout), reinterpret_cast<const bf*>(out), ldo, Dbuf, M, Hq);
     const unsigned block = 256;
-    dim3 gq(static_cast<unsigned>((M + 63) / 64), Hq * TB_HD / 64), gk(static_cast<unsigned>((M + 63) / 64), Hkv * TB_HD / 64);
+    dim3 gq(static_cast<unsigned>((M + 63) / 64), Hq * HD / 64), gk(static_cast<unsigned>((M + 63) / 64), Hkv * HD / 64);
     attn_tc_transpose_kernel<<<gq, block, 0, st>>>(reinterpret_cast<const bf*>(qkv), ld, 0, reinterpret_cast<bf*>(qt), M,
-                                                   Hq * TB_HD);
+                                                   Hq * HD);
     attn_tc_transpose_kernel<<<gq, block, 0, st>>>(reinterpret_cast<const bf*>(dout), ldo, 0, reinterpret_cast<bf*>(dot), M,
-                                                   Hq * TB_HD);
-    attn_tc_transpose_kernel<<<gk, block, 0, st>>>(reinterpret_cast<const bf*>(qkv), ld, Hq * TB_HD,
-                                                   reinterpret_cast<bf*>(kt), M, Hkv * TB_HD);
+                                                   Hq * HD);
+    attn_tc_transpose_kernel<<<gk, block, 0, st>>>(reinterpret_cast<const bf*>(qkv), ld, Hq * HD,
+                                                   reinterpret_cast<bf*>(kt), M, Hkv * HD);
   }
   CUtensorMap tmQKV128, tmQKV64, tmDO128, tmDO64, tmQt, tmDOt, tmKt;
   int e;
-  const uint64_t W = static_cast<uint64_t>(Hq + 2 * Hkv) * TB_HD;
+  const uint64_t W = static_cast<uint64_t>(Hq + 2 * Hkv) * HD;
   if ((e = make_tmap_bf16_2d(&tmQKV128, qkv, M, W, ld, 128, 64))) return e;
   if ((e = make_tmap_bf16_2d(&tmQKV64, qkv, M, W, ld, 64, 64))) return e;
-  if ((e = make_tmap_bf16_2d(&tmDO128, dout, M, static_cast<uint64_t>(Hq) * TB_HD, ldo, 128, 64))) return e;
-  if ((e = make_tmap_bf16_2d(&tmDO64, dout, M, static_cast<uint64_t>(Hq) * TB_HD, ldo, 64, 64))) return e;
-  if ((e = make_tmap_bf16_2d(&tmQt, qt, static_cast<uint64_t>(Hq) * TB_HD, M, M, 128, 64))) return e;
-  if ((e = make_tmap_bf16_2d(&tmDOt, dot, static_cast<uint64_t>(Hq) * TB_HD, M, M, 128, 64))) return e;
-  if ((e = make_tmap_bf16_2d(&tmKt, kt, static_cast<uint64_t>(Hkv) * TB_HD, M, M, 128, 64))) return e;
+  if ((e = make_tmap_bf16_2d(&tmDO128, dout, M, static_cast<uint64_t>(Hq) * HD, ldo, 128, 64))) return e;
+  if ((e = make_tmap_bf16_2d(&tmDO64, dout, M, static_cast<uint64_t>(Hq) * HD, ldo, 64, 64))) return e;
+  if ((e = make_tmap_bf16_2d(&tmQt, qt, static_cast<uint64_t>(Hq) * HD, M, M, HD, 64))) return e;
+  if ((e = make_tmap_bf16_2d(&tmDOt, dot, static_cast<uint64_t>(Hq) * HD, M, M, HD, 64))) return e;
+  if ((e = make_tmap_bf16_2d(&tmKt, kt, static_cast<uint64_t>(Hkv) * HD, M, M, HD, 64))) return e;
+  auto dkv = attn_tc_dkv_kernel<HD>;
+  auto dq = attn_tc_dq_kernel<HD>;
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!configured[dev & 63]) {
-    cudaError_t ce = cudaFuncSetAttribute(attn_tc_dkv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DkvSmem::TOTAL);
+    cudaError_t ce = cudaFuncSetAttribute(dkv, cudaFuncAttributeMaxDynamicSharedMemorySize, DkvSmem<HD>::TOTAL);
     if (ce != cudaSuccess) return static_cast<int>(ce);
-    ce = cudaFuncSetAttribute(attn_tc_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DqSmem::TOTAL);
+    ce = cudaFuncSetAttribute(dq, cudaFuncAttributeMaxDynamicSharedMemorySize, DqSmem<HD>::TOTAL);
     if (ce != cudaSuccess) return static_cast<int>(ce);
     configured[dev & 63] = true;
   }
-  const float scale = 1.f / sqrtf(static_cast<float>(TB_HD));
+  const float scale = 1.f / sqrtf(static_cast<float>(HD));
   const float scale_log2 = 1.4426950408889634f * scale;
-  // split the query heads of a group over two CTAs when a group has at least four heads and the caller gave scratch
-  const int GS = (partial != nullptr && Hq / Hkv >= 4) ? 2 : 1;
   dim3 g1(S / 128, Hkv * GS, rows), g2(S / 128, Hq, rows);
-  attn_tc_dkv_kernel<<<g1, TB_THREADS, DkvSmem::TOTAL, st>>>(tmQKV128, tmQKV64, tmDO64, tmQt, tmDOt, gid, pid, state, lse2,
-                                                            Dbuf, reinterpret_cast<bf*>(dqkv), ld, S, Hq, Hkv, scale,
-                                                            scale_log2, M, GS, GS > 1 ? partial : nullptr, status);
+  dkv<<<g1, TB_THREADS, DkvSmem<HD>::TOTAL, st>>>(tmQKV128, tmQKV64, tmDO64, tmQt, tmDOt, gid, pid, state, lse2, Dbuf,
+                                                  reinterpret_cast<bf*>(dqkv), ld, S, Hq, Hkv, scale, scale_log2, M, GS,
+                                                  GS > 1 ? partial : nullptr, status);
   if (GS > 1) {
-    const long total = M * ((2 * Hkv * TB_HD) >> 2);
+    const long total = M * ((2 * Hkv * HD) >> 2);
     attn_tc_combine_dkv_kernel<<<static_cast<unsigned>(std::min<long>((total + 255) / 256, 148 * 16)), 256, 0, st>>>(
-        partial, GS, reinterpret_cast<bf*>(dqkv), ld, Hq * TB_HD, M, Hkv * TB_HD, scale);
+        partial, GS, reinterpret_cast<bf*>(dqkv), ld, Hq * HD, M, Hkv * HD, scale);
   }
-  attn_tc_dq_kernel<<<g2, TB_THREADS, DqSmem::TOTAL, st>>>(tmQKV128, tmQKV64, tmDO128, tmKt, gid, pid, state, lse2, Dbuf,
-                                                          reinterpret_cast<bf*>(dqkv), ld, S, Hq, Hkv, scale, scale_log2,
-                                                          M, status);
+  dq<<<g2, TB_THREADS, DqSmem<HD>::TOTAL, st>>>(tmQKV128, tmQKV64, tmDO128, tmKt, gid, pid, state, lse2, Dbuf,
+                                                reinterpret_cast<bf*>(dqkv), ld, S, Hq, Hkv, scale, scale_log2, M, status);
   return static_cast<int>(cudaGetLastError());
+}
+
+}  // namespace artb
+
+// How many CTAs share the query heads of a kv group in the dK / dV kernel.  The key blocks at the start of a row see every
+// later query, so that with one CTA per (block, kv head) they are the critical path; two per group from four heads on, and
+// more while the grid is below two per SM (a single 2048-token row has 16 blocks x 2 to 4 kv heads).
+ARTB_EXPORT int artb_attn_tc_bwd_splits(int rows, int S, int Hq, int Hkv) {
+  const int G = Hq / Hkv;
+  const long ctas = static_cast<long>(S / 128) * Hkv * rows;
+  int gs = G >= 4 ? 2 : 1;
+  while (gs < G && ctas * gs < 2L * sm_count()) ++gs;
+  const int per = (G + gs - 1) / gs;
+  return (G + per - 1) / per;      // no CTA without heads
+}
+
+// qkv / dqkv [rows*S, ld] (q | k | v columns); out, dout [rows*S, ldo]; lse2, Dbuf fp32 [Hq, rows*S];
+// scratch bf16: qt, dot [Hq*hd, rows*S], kt [Hkv*hd, rows*S]; partial: fp32 [splits, rows*S, 2*Hkv*hd] when the kv groups
+// are split (artb_attn_tc_bwd_splits).  Head dim 64 or 128, S % 128 == 0.
+ARTB_EXPORT int artb_attn_tc_bwd(const void* qkv, int ld, const void* out, const void* dout, int ldo, const int* gid,
+                                 const int* pid, const uint8_t* state, const float* lse2, float* Dbuf, void* qt, void* dot,
+                                 void* kt, void* dqkv, float* partial, int splits, int rows, int S, int Hq, int Hkv, int hd,
+                                 int* status, cudaStream_t st) {
+  if (S % 128 || Hq % Hkv || (ld & 7) || (ldo & 7) || (splits > 1 && !partial)) return ERR_BAD_SHAPE;
+  if (splits < 1 || splits > Hq / Hkv || static_cast<long>(rows) * S > 0x7fffffffL) return ERR_BAD_SHAPE;
+  auto go = hd == 128 ? launch_tc_bwd<128> : hd == 64 ? launch_tc_bwd<64> : nullptr;
+  if (!go) return ERR_BAD_SHAPE;
+  return go(qkv, ld, out, dout, ldo, gid, pid, state, lse2, Dbuf, qt, dot, kt, dqkv, partial, splits, rows, S, Hq, Hkv, status,
+            st);
 }

@@ -15,7 +15,8 @@ _sigs = {
     "artb_attn_tree_fwd": [vp, ci, vp, vp, vp, vp, ci, vp, ci, ci, ci, ci, ci, vp],
     "artb_attn_tree_bwd": [vp, ci, vp, vp, ci, vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, ci, ci, vp],
     "artb_attn_tc_fwd": [vp, ci, vp, vp, vp, vp, vp, ci, vp, ci, ci, ci, ci, vp, vp],
-    "artb_attn_tc_bwd": [vp, ci, vp, vp, ci, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, ci, vp, vp],
+    "artb_attn_tc_bwd": [vp, ci, vp, vp, ci, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, ci, ci, ci, vp, vp],
+    "artb_attn_tc_bwd_splits": [ci, ci, ci, ci],
 }
 # forward on tcgen05 / TMEM when the shape allows it (head dim 128, rows a multiple of 128 tokens)
 USE_TC = os.environ.get("ARTB_ATTN_TC", "1") == "1"
@@ -66,15 +67,18 @@ def backward(dout: torch.Tensor, saved: tuple, plan) -> torch.Tensor:
     M, S = qkv.shape[0], plan.S
     dqkv = torch.empty_like(qkv)
     dbuf = torch.empty((Hq, M), dtype=torch.float32, device=qkv.device)
-    if USE_TC_BWD and hd == 128 and S % 128 == 0 and M % 8 == 0:
+    # tcgen05: at head dim 64 its two kernels replace one that adds fp32 dQ rows with atomics (1027 us against 119 us with all
+    # helpers, 14 / 2 heads and a 2048-token row); the forward of that size stays with the mma.sync kernel, 33 us
+    if USE_TC_BWD and hd in (64, 128) and S % 128 == 0 and M % 8 == 0:
         qt = torch.empty((Hq * hd, M), dtype=qkv.dtype, device=qkv.device)
         dot = torch.empty((Hq * hd, M), dtype=qkv.dtype, device=qkv.device)
         kt = torch.empty((Hkv * hd, M), dtype=qkv.dtype, device=qkv.device)
-        partial = torch.empty((2, M, 2 * Hkv * hd), dtype=torch.float32, device=qkv.device) if Hq // Hkv >= 4 else None
+        splits = _f("artb_attn_tc_bwd_splits")(M // S, S, Hq, Hkv)
+        partial = torch.empty((splits, M, 2 * Hkv * hd), dtype=torch.float32, device=qkv.device) if splits > 1 else None
         _lib.check_rc(_f("artb_attn_tc_bwd")(_lib.ptr(qkv), qkv.stride(0), _lib.ptr(out), _lib.ptr(dout), out.stride(0),
                                              _lib.ptr(plan.gid), _lib.ptr(plan.pid), _lib.ptr(plan.state),
                                              _lib.ptr(lse2), _lib.ptr(dbuf), _lib.ptr(qt), _lib.ptr(dot), _lib.ptr(kt),
-                                             _lib.ptr(dqkv), _lib.ptr(partial), M // S, S, Hq, Hkv,
+                                             _lib.ptr(dqkv), _lib.ptr(partial), splits, M // S, S, Hq, Hkv, hd,
                                              _lib.ptr(_lib.status_word(qkv.device)), _lib.stream_ptr()), "attn_tc_bwd")
         return dqkv
     dq_acc = torch.empty((M, Hq * hd), dtype=torch.float32, device=qkv.device)
