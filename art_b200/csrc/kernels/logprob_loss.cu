@@ -21,6 +21,8 @@
 // src/art/local/train.py:245-281 and the loss arithmetic at src/art/local/train.py:112-151.
 #include <math.h>
 
+#include <type_traits>
+
 #include "gemm_pipeline_2cta.cuh"
 #include "host_utils.h"
 #include "sampling.cuh"
@@ -52,9 +54,30 @@ struct SchedVocabSplit {
   }
 };
 
+// Schedule of the decode-time sampler: one item (128 rows, a span of n-tiles) per CTA, the spans as equal as whole tiles
+// allow.  With a fixed number of tiles per split and two items per CTA the longest CTA of a 152 064-token head had 6 tiles
+// of 256 where the mean is 4.0.
+struct SchedVocabSpan {
+  int m_tiles, n_tiles, splits;
+  __device__ int lo(int s) const { return static_cast<int>(static_cast<long>(s) * n_tiles / splits); }
+  __device__ int tiles_for_cta(int cta, int) const {
+    const int s = cta / m_tiles;
+    return s < splits ? lo(s + 1) - lo(s) : 0;
+  }
+  __device__ TileInfo get(int cta, int, int i) const {
+    const int s = cta / m_tiles, first = lo(s), end = lo(s + 1);
+    TileInfo ti = make_tile(cta % m_tiles, first + i);
+    ti.group = s;
+    ti.first = i == 0;
+    ti.last = first + i == end - 1;
+    return ti;
+  }
+};
+
 struct EpiStats {
+  static constexpr int COL_SPLIT = 2;   // two warps per lane quarter, each with a partial of its own for its half of the columns
   const int* target;   // [M] target vocabulary id per row (global id, minus vocab_offset locally)
-  float* partials;     // [splits, M, 4]  (max, sumexp, z_target, unused)
+  float* partials;     // [2 splits, M, 4]  (max, sumexp, z_target, unused)
   float* logits;       // [M, ldl] fp32, or null: not kept
   int M, V, ldl, vocab_offset;
   float run_max, run_sum, z;
@@ -72,13 +95,7 @@ struct EpiStats {
   __device__ void chunk(const TileInfo& ti, int row, int c, uint32_t (&acc)[32]) {
     const int gc = ti.n_blk * LP_BN + c;
     if (gc >= V) return;
-    const int gr = ti.m_blk * GEMM_BM + row;
-    if (logits && gr < M) {
-      float* o = logits + static_cast<size_t>(gr) * ldl + gc;
-#pragma unroll
-      for (int j = 0; j < 32; j += 4)
-        if (gc + j < ldl) *reinterpret_cast<uint4*>(o + j) = make_uint4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
-    }
+    if (logits) store_logits(ti, row, gc, acc);
     float cmax = -INFINITY;
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
@@ -100,12 +117,31 @@ struct EpiStats {
         if (j == d) z = __uint_as_float(acc[j]);
     }
   }
+  // 32 rows x 128 bytes of a warp, turned in shared memory so that a store covers whole lines of 4 rows: with a row per lane
+  // every store touched 32 lines, and on a K of 896 the tile's main loop is shorter than that (692 us for 1734 rows of the
+  // 151 936-token head, against 396 without stores).  Piece p of row r sits at r * 8 + (p ^ (r & 7)): no bank conflicts.
+  __device__ __forceinline__ void store_logits(const TileInfo& ti, int row, int gc, const uint32_t (&acc)[32]) {
+    __shared__ uint4 s_slab[8][32 * 8];
+    const int lane = row & 31, sw = lane & 7;
+    uint4* sb = s_slab[epi_warp_slot()];
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sb[lane * 8 + (j ^ sw)] = make_uint4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
+    __syncwarp();
+    const int row0 = ti.m_blk * GEMM_BM + (row & ~31), col = gc + 4 * sw;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = i * 4 + (lane >> 3);
+      if (row0 + r < M && col < ldl)
+        *reinterpret_cast<uint4*>(logits + static_cast<size_t>(row0 + r) * ldl + col) = sb[r * 8 + (sw ^ (r & 7))];
+    }
+  }
   __device__ void tile_end(const TileInfo& ti, int row) {
     if (!ti.last) return;
     const int gr = ti.m_blk * GEMM_BM + row;
     if (gr >= M) return;
     float4 o = make_float4(run_max, run_sum, z, 0.f);
-    *reinterpret_cast<float4*>(partials + (static_cast<size_t>(ti.group) * M + gr) * 4) = o;
+    *reinterpret_cast<float4*>(partials + (static_cast<size_t>(ti.group * 2 + (epi_warp_slot() >> 2)) * M + gr) * 4) = o;
   }
 };
 
@@ -164,8 +200,12 @@ struct EpiDLogits {
 // log-probability under the sampling distribution without materialising logits.
 //   x = logit * inv_temp ;  sample = argmax_v (x_v + g_v),  g_v = -log(-log(u_v)),  u_v = hash(seed, row, v)
 // inv_temp == 0 selects greedy decoding (argmax of the raw logits, log-prob at temperature 1).
+// Noise, exponential and arg-max are some 40 dependent instructions per logit: two warps per lane quarter, each with the
+// statistics of its half of every tile's columns (a partial of its own).
+template <int BN>
 struct EpiSample {
-  float* partials;        // [splits, M, 8]: max, sumexp, best_score, best_idx(bits), best_x, -, -, -
+  static constexpr int COL_SPLIT = 2;
+  float* partials;        // [2 splits, M, 8]: max, sumexp, best_score, best_idx(bits), best_x, -, -, -
   const float* inv_temp;  // [M] per-row 1/temperature (0 = greedy)
   const uint32_t* row_seed;  // [M] per-row seed (request seed mixed with the decode step)
   int M, V, vocab_offset;
@@ -186,7 +226,7 @@ struct EpiSample {
     }
   }
   __device__ void chunk(const TileInfo& ti, int row, int c, uint32_t (&acc)[32]) {
-    const int gc = ti.n_blk * LP_BN + c;
+    const int gc = ti.n_blk * BN + c;
     if (gc >= V) return;
     const uint32_t gr = ti.m_blk * GEMM_BM + row;
     const bool greedy = it == 0.f;
@@ -220,7 +260,7 @@ struct EpiSample {
     if (!ti.last) return;
     const int gr = ti.m_blk * GEMM_BM + row;
     if (gr >= M) return;
-    float* o = partials + (static_cast<size_t>(ti.group) * M + gr) * 8;
+    float* o = partials + (static_cast<size_t>(ti.group * 2 + (epi_warp_slot() >> 2)) * M + gr) * 8;
     *reinterpret_cast<float4*>(o) = make_float4(run_max, run_sum, best_score, __int_as_float(best_idx));
     *reinterpret_cast<float4*>(o + 4) = make_float4(best_x, 0.f, 0.f, 0.f);
   }
@@ -228,25 +268,46 @@ struct EpiSample {
 
 // Merge sampling partials (over vocabulary splits and, for tensor-parallel heads, over ranks'
 // partial buffers laid out back to back): token id and log-prob per row.
+// One warp per row: a thread per row walked 200 to 300 partials one after another, 20 to 45 us.
 __global__ void sample_merge_kernel(const float* __restrict__ partials, int parts, int M, int* __restrict__ token,
                                     float* __restrict__ logprob) {
-  const int tI = blockIdx.x * blockDim.x + threadIdx.x;
-  if (tI >= M) return;
-  float mx = -INFINITY;
-  for (int s = 0; s < parts; ++s) mx = fmaxf(mx, partials[(static_cast<size_t>(s) * M + tI) * 8]);
-  float sum = 0.f, best = -INFINITY, bx = 0.f;
-  int bi = -1;
-  for (int s = 0; s < parts; ++s) {
-    const float* p = partials + (static_cast<size_t>(s) * M + tI) * 8;
-    sum += p[1] * __expf(p[0] - mx);
-    if (p[2] > best) {
-      best = p[2];
-      bi = __float_as_int(p[3]);
-      bx = p[4];
+  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (row >= M) return;
+  float mx = -INFINITY, sum = 0.f, best = -INFINITY, bx = 0.f;
+  int bi = -1, bs = 0x7fffffff;
+  for (int s = lane; s < parts; s += 32) {
+    const float4* p = reinterpret_cast<const float4*>(partials + (static_cast<size_t>(s) * M + row) * 8);
+    const float4 a = p[0];
+    const float x = p[1].x;
+    const float n = fmaxf(mx, a.x);
+    if (n != -INFINITY) sum = sum * __expf(mx - n) + a.y * __expf(a.x - n);
+    mx = n;
+    if (a.z > best) {
+      best = a.z;
+      bi = __float_as_int(a.w);
+      bx = x;
+      bs = s;
     }
   }
-  token[tI] = bi;
-  logprob[tI] = bx - (mx + logf(sum));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float m2 = __shfl_xor_sync(0xffffffffu, mx, o), s2 = __shfl_xor_sync(0xffffffffu, sum, o);
+    const float b2 = __shfl_xor_sync(0xffffffffu, best, o), x2 = __shfl_xor_sync(0xffffffffu, bx, o);
+    const int i2 = __shfl_xor_sync(0xffffffffu, bi, o), p2 = __shfl_xor_sync(0xffffffffu, bs, o);
+    const float n = fmaxf(mx, m2);
+    if (n != -INFINITY) sum = sum * __expf(mx - n) + s2 * __expf(m2 - n);
+    mx = n;
+    if (b2 > best || (b2 == best && p2 < bs)) {      // ties: the first partial, as in one pass
+      best = b2;
+      bi = i2;
+      bx = x2;
+      bs = p2;
+    }
+  }
+  if (lane == 0) {
+    token[row] = bi;
+    logprob[row] = bx - (mx + logf(sum));
+  }
 }
 
 // Merge vocabulary-split partials and evaluate the per-token GRPO terms.
@@ -431,8 +492,8 @@ static int launch_lp(const void* H, int ldh, const void* W, int ldw, int M, int 
 using namespace artb;
 
 // Number of vocabulary splits the forward uses for (M, V): enough (m_blk, split) items to
-// fill the machine, never more splits than n-tiles.  The partials buffer is [splits, M, 4] fp32.
-ARTB_EXPORT int artb_logprob_splits(int M, int V) {
+// fill the machine, never more splits than n-tiles.
+static int lp_splits(int M, int V) {
   const bool pairs = lp_pairs(M);
   const int m_tiles = pairs ? (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM) : (M + GEMM_BM - 1) / GEMM_BM;
   const int n_tiles = (V + LP_BN - 1) / LP_BN;
@@ -445,12 +506,15 @@ ARTB_EXPORT int artb_logprob_splits(int M, int V) {
   return splits;
 }
 
+// The partials buffer of artb_logprob_partials is [artb_logprob_parts, M, 4] fp32: two per split.
+ARTB_EXPORT int artb_logprob_parts(int M, int V) { return 2 * lp_splits(M, V); }
+
 // Phase 1: per-split online-softmax partials over the vocabulary shard W[V, K]; with `logits` ([M, ldl] fp32, ldl >= V and a
 // multiple of 8) the logits are kept for artb_dlogits_inplace.
 ARTB_EXPORT int artb_logprob_partials(const void* H, int ldh, const void* W, int ldw, const int* target,
-                                      float* partials, float* logits, int ldl, int M, int V, int K, int splits,
+                                      float* partials, float* logits, int ldl, int M, int V, int K, int parts,
                                       int vocab_offset, int* status, cudaStream_t stream) {
-  if (M <= 0 || V <= 0 || (K & 7) || (logits && (ldl < V || (ldl & 7)))) return ERR_BAD_SHAPE;
+  if (M <= 0 || V <= 0 || (K & 7) || parts != artb_logprob_parts(M, V) || (logits && (ldl < V || (ldl & 7)))) return ERR_BAD_SHAPE;
   if (reinterpret_cast<uintptr_t>(logits) & 15) return ERR_BAD_ALIGN;
   EpiStats epi;
   epi.target = target;
@@ -464,7 +528,7 @@ ARTB_EXPORT int artb_logprob_partials(const void* H, int ldh, const void* W, int
   epi.run_sum = 0.f;
   epi.z = 0.f;
   epi.tgt = -1;
-  return launch_lp(H, ldh, W, ldw, M, V, K, splits, epi, status, stream);
+  return launch_lp(H, ldh, W, ldw, M, V, K, parts / 2, epi, status, stream);
 }
 
 // Phase 2: merge partials -> lse, logprob; GRPO terms; coef = dLoss/dlogprob.
@@ -500,7 +564,7 @@ ARTB_EXPORT int artb_logprob_dlogits(const void* H, int ldh, const void* W, int 
   epi.tgt = -1;
   // one split per n-tile group is irrelevant here (no cross-tile state): reuse the
   // vocab-split schedule so LM-head tiles are shared through L2 the same way.
-  int splits = artb_logprob_splits(M, V);
+  int splits = lp_splits(M, V);
   return launch_lp(H, ldh, W, ldw, M, V, K, splits, epi, status, stream);
 }
 
@@ -514,12 +578,12 @@ ARTB_EXPORT int artb_dlogits_inplace(float* buf, int ldl, const int* target, con
   return static_cast<int>(cudaGetLastError());
 }
 
-// Rollout sampling: partials [splits, M, 8] for one vocabulary shard (see EpiSample).
-ARTB_EXPORT int artb_sample_partials(const void* H, int ldh, const void* W, int ldw, const float* inv_temp,
-                                     const uint32_t* row_seed, float* partials, int M, int V, int K, int splits,
-                                     int vocab_offset, int* status, cudaStream_t stream) {
-  if (M <= 0 || V <= 0 || (K & 7)) return ERR_BAD_SHAPE;
-  EpiSample epi;
+namespace artb {
+
+template <int BN>
+static EpiSample<BN> sample_epi(const float* inv_temp, const uint32_t* row_seed, float* partials, int M, int V,
+                                int vocab_offset) {
+  EpiSample<BN> epi;
   epi.partials = partials;
   epi.inv_temp = inv_temp;
   epi.row_seed = row_seed;
@@ -529,12 +593,79 @@ ARTB_EXPORT int artb_sample_partials(const void* H, int ldh, const void* W, int 
   epi.run_max = epi.run_sum = epi.best_score = epi.best_x = epi.it = 0.f;
   epi.best_idx = -1;
   epi.seed = 0;
-  return launch_lp(H, ldh, W, ldw, M, V, K, splits, epi, status, stream);
+  return epi;
+}
+
+// Decode batches (below the CTA-pair limit): vocabulary spans of whole BN-wide tiles, one per CTA.
+struct SamplePlan {
+  int bn, n_tiles, m_tiles, splits;
+};
+// The tile width of 256, 224 or 160 columns whose longest span is the shortest, the widest where they tie: 152 064 tokens
+// over 148 CTAs are 5 x 224 columns (the mean is 1027; 5 x 256 would be 14 % more), over 74 (129 to 256 rows) 13 x 160.
+static SamplePlan sample_plan(int M, int V) {
+  SamplePlan best{0, 0, 0, 0};
+  long cost = 0;
+  for (int bn : {256, 224, 160}) {
+    SamplePlan p{bn, (V + bn - 1) / bn, (M + GEMM_BM - 1) / GEMM_BM, 0};
+    p.splits = sm_count() / p.m_tiles;
+    if (p.splits > p.n_tiles) p.splits = p.n_tiles;
+    if (p.splits < 1) p.splits = 1;
+    const long c = static_cast<long>((p.n_tiles + p.splits - 1) / p.splits) * bn;
+    if (best.bn == 0 || c < cost) {
+      best = p;
+      cost = c;
+    }
+  }
+  return best;
+}
+
+template <int BN, int STAGES>
+static int launch_sample(const void* H, int ldh, const void* W, int ldw, const SamplePlan& p, const EpiSample<BN>& epi, int K,
+                         int* status, cudaStream_t stream) {
+  using L = GemmSmemLayout<BN, STAGES>;
+  static_assert(L::TOTAL <= 227 * 1024, "shared memory");
+  CUtensorMap tA, tB;
+  int rc;
+  if ((rc = make_tmap_bf16_2d(&tA, H, epi.M, K, ldh, GEMM_BM, GEMM_BK))) return rc;
+  if ((rc = make_tmap_bf16_2d(&tB, W, epi.V, K, ldw, BN, GEMM_BK))) return rc;
+  auto kern = gemm_tcgen05_kernel<BN, STAGES, SchedVocabSpan, EpiSample<BN>>;
+  static bool configured[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!configured[dev & 63]) {
+    cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
+    if (ce != cudaSuccess) return static_cast<int>(ce);
+    configured[dev & 63] = true;
+  }
+  const SchedVocabSpan sched{p.m_tiles, p.n_tiles, p.splits};
+  return static_cast<int>(launch_kernel(kern, dim3(p.m_tiles * p.splits), dim3(gemm_pipe_threads<EpiSample<BN>>()), L::TOTAL,
+                                        stream, tA, tB, tA, tB, (K + GEMM_BK - 1) / GEMM_BK, 0, sched, epi, status, NoComm{}));
+}
+
+}  // namespace artb
+
+// Partials of artb_sample_partials for (M, V): two per vocabulary split.
+ARTB_EXPORT int artb_sample_parts(int M, int V) {
+  return 2 * (lp_pairs(M) ? lp_splits(M, V) : sample_plan(M, V).splits);
+}
+
+// Rollout sampling: partials [parts, M, 8] for one vocabulary shard (see EpiSample), parts = artb_sample_parts(M, V).
+ARTB_EXPORT int artb_sample_partials(const void* H, int ldh, const void* W, int ldw, const float* inv_temp,
+                                     const uint32_t* row_seed, float* partials, int M, int V, int K, int parts,
+                                     int vocab_offset, int* status, cudaStream_t stream) {
+  if (M <= 0 || V <= 0 || (K & 7) || parts != artb_sample_parts(M, V)) return ERR_BAD_SHAPE;
+  auto epi = [&](auto bn) { return sample_epi<decltype(bn)::value>(inv_temp, row_seed, partials, M, V, vocab_offset); };
+  using W256 = std::integral_constant<int, 256>;
+  if (lp_pairs(M)) return launch_lp(H, ldh, W, ldw, M, V, K, parts / 2, epi(W256{}), status, stream);
+  const SamplePlan p = sample_plan(M, V);
+  if (p.bn == 256) return launch_sample<256, 4>(H, ldh, W, ldw, p, epi(W256{}), K, status, stream);
+  if (p.bn == 224) return launch_sample<224, 5>(H, ldh, W, ldw, p, epi(std::integral_constant<int, 224>{}), K, status, stream);
+  return launch_sample<160, 6>(H, ldh, W, ldw, p, epi(std::integral_constant<int, 160>{}), K, status, stream);
 }
 
 ARTB_EXPORT int artb_sample_merge(const float* partials, int parts, int M, int* token, float* logprob,
                                   cudaStream_t stream) {
   if (M <= 0) return 0;
-  sample_merge_kernel<<<(M + 127) / 128, 128, 0, stream>>>(partials, parts, M, token, logprob);
+  sample_merge_kernel<<<(M + 3) / 4, 128, 0, stream>>>(partials, parts, M, token, logprob);
   return static_cast<int>(cudaGetLastError());
 }

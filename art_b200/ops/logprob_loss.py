@@ -17,7 +17,7 @@ from .gemm import gemm_tn
 vp, ci, cf = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
 _bound: dict[str, object] = {}
 _sigs = {
-    "artb_logprob_splits": [ci, ci],
+    "artb_logprob_parts": [ci, ci],
     "artb_logprob_partials": [vp, ci, vp, ci, vp, vp, vp, ci, ci, ci, ci, ci, ci, vp, vp],
     "artb_dlogits_inplace": [vp, ci, vp, vp, vp, ci, ci, ci, vp],
     "artb_grpo_tokens": [vp, ci, ci, vp, vp, vp, vp, cf, cf, cf, vp, vp, vp, vp, vp],
@@ -45,18 +45,18 @@ class LogprobResult:
 
 def partials(hidden: torch.Tensor, lm_head: torch.Tensor, target: torch.Tensor, vocab_offset: int = 0,
              logits: torch.Tensor | None = None) -> tuple[torch.Tensor, int]:
-    """Per-vocab-split (max, sumexp, z_target) for one vocabulary shard: [splits, M, 4] fp32.  ``logits`` ([M, ldl] fp32,
+    """Partial (max, sumexp, z_target) of one vocabulary shard: [parts, M, 4] fp32, and ``parts``.  ``logits`` ([M, ldl] fp32,
     ``ldl`` a multiple of 8) also receives the logits."""
     M, K = hidden.shape
     V = lm_head.shape[0]
-    splits = _f("artb_logprob_splits")(M, V)
-    part = torch.empty((splits, M, 4), dtype=torch.float32, device=hidden.device)
+    parts = _f("artb_logprob_parts")(M, V)
+    part = torch.empty((parts, M, 4), dtype=torch.float32, device=hidden.device)
     rc = _f("artb_logprob_partials")(_lib.ptr(hidden), hidden.stride(0), _lib.ptr(lm_head), lm_head.stride(0),
                                      _lib.ptr(target), _lib.ptr(part), _lib.ptr(logits),
-                                     logits.stride(0) if logits is not None else 0, M, V, K, splits, vocab_offset,
+                                     logits.stride(0) if logits is not None else 0, M, V, K, parts, vocab_offset,
                                      _lib.ptr(_lib.status_word(hidden.device)), _lib.stream_ptr())
     _lib.check_rc(rc, "logprob_partials")
-    return part, splits
+    return part, parts
 
 
 def grpo_tokens(part: torch.Tensor, old_lp=None, adv=None, tok_w=None, ref_lp=None, eps_lo: float = 0.2,

@@ -17,7 +17,7 @@ _sigs = {
     "artb_decode_advance": [vp, vp, vp, vp, vp, vp, ci, ci, vp, ci, vp],
     "artb_sample_partials": [vp, ci, vp, ci, vp, vp, vp, ci, ci, ci, ci, ci, vp, vp],
     "artb_sample_merge": [vp, ci, ci, vp, vp, vp],
-    "artb_logprob_splits": [ci, ci],
+    "artb_sample_parts": [ci, ci],
     "artb_sample_restricted": [vp, cl, vp, vp, vp, vp, vp, ci, ci, ci, vp, vp, vp],
     "artb_logit_adjust": [vp, cl, vp, vp, vp, vp, vp, ci, ci, ci, vp],
     "artb_top_logprobs": [vp, cl, vp, ci, ci, ci, vp, vp, vp],
@@ -126,15 +126,15 @@ def decode_advance(sampled, tokens, pos, ctx_len, slot, block_table, block_size:
 
 def sample_partials(hidden: torch.Tensor, lm_head: torch.Tensor, inv_temp: torch.Tensor, row_seed: torch.Tensor,
                     vocab_offset: int = 0) -> torch.Tensor:
-    """Sampling statistics of one vocabulary shard: ``[splits, M, 8]`` fp32 (running max, sum of exponentials, best
+    """Sampling statistics of one vocabulary shard: ``[parts, M, 8]`` fp32 (running max, sum of exponentials, best
     perturbed score with its index and logit).  Partials of different shards concatenate along dim 0 and
     :func:`sample_merge` reduces them, which is all a vocabulary-parallel LM head has to exchange."""
     M, K = hidden.shape
     V = lm_head.shape[0]
-    splits = _f("artb_logprob_splits")(M, V)
-    part = torch.empty((splits, M, 8), dtype=torch.float32, device=hidden.device)
+    parts = _f("artb_sample_parts")(M, V)
+    part = torch.empty((parts, M, 8), dtype=torch.float32, device=hidden.device)
     _lib.check_rc(_f("artb_sample_partials")(_lib.ptr(hidden), hidden.stride(0), _lib.ptr(lm_head), lm_head.stride(0),
-                                             _lib.ptr(inv_temp), _lib.ptr(row_seed), _lib.ptr(part), M, V, K, splits,
+                                             _lib.ptr(inv_temp), _lib.ptr(row_seed), _lib.ptr(part), M, V, K, parts,
                                              vocab_offset, _lib.ptr(_lib.status_word(hidden.device)),
                                              _lib.stream_ptr()), "sample_partials")
     return part
