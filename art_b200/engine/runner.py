@@ -917,13 +917,13 @@ class NativeRunner(DeviceRunner):
                 h, _ = ew.rmsnorm_fwd(x, self.layers[0]["ln1"], cfg.rms_norm_eps, want_rstd=False)
                 for li, L in enumerate(self.layers):
                     nxt = self.layers[li + 1]["ln1"] if li + 1 < len(self.layers) else self.final_norm
-                    x, h = self._layer_decode_fused(li, L, x, h, nxt, st, any_lora, splits, ws)
+                    x, h = self._layer_decode_fused(li, L, x, h, nxt, st, any_lora)
                 hidden = h
             else:
                 for li, L in enumerate(self.layers):
                     qkv = self._qkv(L, x, st["pos"], st["ad"], any_lora)
                     paged.kv_write(qkv, cfg.q_size, cfg.q_size + cfg.kv_size, st["slot"], self.kv.k[li], self.kv.v[li])
-                    paged.paged_decode(qkv, self.kv.k[li], self.kv.v[li], st["bt"], st["ctx"], Hq, Hkv, hd, st["attn_out"], splits, ws)
+                    paged.paged_decode_even(qkv, self.kv.k[li], self.kv.v[li], st["bt"], st["ctx"], Hq, Hkv, hd, st["attn_out"], st["attn_ws"])
                     x2 = self._reduce(L["o"](st["attn_out"], st["ad"], any_lora, residual=self._res(x)))
                     x = self._mlp(L, x2, st["ad"], any_lora)
                 hidden, _ = ew.rmsnorm_fwd(x, self.final_norm, cfg.rms_norm_eps, want_rstd=False)
@@ -944,7 +944,7 @@ class NativeRunner(DeviceRunner):
         L = self.layers[0]
         return all(isinstance(L.get(k), EngineLinear) and L[k].cols <= 64 for k in ("qkv", "o", "gu", "down"))
 
-    def _layer_decode_fused(self, li: int, L, x, h, next_norm, st, any_lora: bool, splits: int, ws):
+    def _layer_decode_fused(self, li: int, L, x, h, next_norm, st, any_lora: bool):
         from ..ops import paged
 
         cfg = self.cfg
@@ -956,7 +956,7 @@ class NativeRunner(DeviceRunner):
         paged.decode_finalize_qkv(w, M, Hq, Hkv, hd, lin.kpad, st["pos"], cfg.rope_theta, st["slot"], self.kv.k[li],
                                   self.kv.v[li], st["q"], bias=None if lin.bias_ext is None else lin.bias_ext[:lin.N],
                                   adapter=ad, B_all=lin.B_T, cols=lin.cols)
-        paged.paged_decode(st["q"], self.kv.k[li], self.kv.v[li], st["bt"], st["ctx"], Hq, Hkv, hd, st["attn_out"], splits, ws)
+        paged.paged_decode_even(st["q"], self.kv.k[li], self.kv.v[li], st["bt"], st["ctx"], Hq, Hkv, hd, st["attn_out"], st["attn_ws"])
         lin = L["o"]
         w = lin.partial_sums(st["attn_out"], any_lora)
         x2, h2 = torch.empty_like(x), torch.empty_like(x)
@@ -980,12 +980,12 @@ class NativeRunner(DeviceRunner):
         return ew.rmsnorm_fwd(ew.gather_rows(x, rows), self.final_norm, self.cfg.rms_norm_eps, want_rstd=False)[0]
 
     def _decode_buffers(self, nb: int) -> dict:
+        from ..ops import paged
+
         cfg = self.cfg
         return {"attn_out": torch.zeros((nb, cfg.q_size), dtype=torch.bfloat16, device=self.device),
-                "q": torch.zeros((nb, cfg.q_size), dtype=torch.bfloat16, device=self.device)}
+                "q": torch.zeros((nb, cfg.q_size), dtype=torch.bfloat16, device=self.device),
+                "attn_ws": paged.even_decode_workspace(nb, cfg.num_heads, cfg.num_kv_heads, cfg.head_dim, self.device)}
 
     def _attn_splits(self, nb: int, max_ctx: int) -> int:
-        return 1 if nb * self.cfg.num_kv_heads >= 128 else min(8, max(1, 1 << (max(1, max_ctx // 512).bit_length() - 1)))
-
-    def _attn_workspace(self, nb: int, splits: int) -> torch.Tensor:
-        return torch.empty(nb * self.cfg.num_heads * splits * (self.cfg.head_dim + 2), dtype=torch.float32, device=self.device)
+        return 1        # the decode attention shares the keys out by itself, on the device

@@ -12,6 +12,8 @@ vp, ci, cl = ctypes.c_void_p, ctypes.c_int, ctypes.c_long
 _sigs = {
     "artb_kv_write": [vp, ci, ci, ci, vp, vp, vp, ci, ci, cl, vp, vp],
     "artb_kv_gather": [vp, vp, vp, ci, ci, vp, ci, ci, ci, ci, cl, vp, vp],
+    "artb_paged_decode_even": [vp, ci, vp, vp, vp, ci, vp, ci, ci, ci, ci, ci, vp, ci, vp, cl, vp, vp],
+    "artb_paged_decode_even_bytes": [ci, ci, ci, ci],
     "artb_paged_decode": [vp, ci, vp, vp, vp, ci, vp, ci, ci, ci, ci, ci, vp, ci, vp, ci, cl, vp, vp],
     "artb_lora_slot_mask": [vp, ci, vp, cl, ci, ci, vp, vp],
     "artb_decode_advance": [vp, vp, vp, vp, vp, vp, ci, ci, vp, ci, vp],
@@ -108,6 +110,26 @@ def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
                                           n, Hq, Hkv, hd, _lib.ptr(out), out.stride(0), _lib.ptr(ws), splits,
                                           k_cache.shape[0], _lib.ptr(_lib.status_word(q.device)), _lib.stream_ptr()),
                   "paged_decode")
+    return out
+
+
+def even_decode_workspace(n: int, Hq: int, Hkv: int, hd: int, device) -> torch.Tensor:
+    """Workspace of :func:`paged_decode_even` for ``n`` sequences; one call at a time may use it."""
+    return torch.zeros(_f("artb_paged_decode_even_bytes")(n, Hq, Hkv, hd), dtype=torch.uint8, device=device)
+
+
+def paged_decode_even(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,
+                      ctx_len: torch.Tensor, Hq: int, Hkv: int, hd: int, out: torch.Tensor, ws: torch.Tensor) -> torch.Tensor:
+    """:func:`paged_decode` with the keys of all sequences in even shares over the chip, whatever their lengths."""
+    n = q.shape[0]
+    need = _f("artb_paged_decode_even_bytes")(n, Hq, Hkv, hd)
+    if ws.numel() * ws.element_size() < need:
+        raise ValueError(f"workspace of {ws.numel() * ws.element_size()} bytes, {need} needed")
+    _lib.check_rc(_f("artb_paged_decode_even")(_lib.ptr(q), q.stride(0), _lib.ptr(k_cache), _lib.ptr(v_cache),
+                                               _lib.ptr(block_table), block_table.stride(0), _lib.ptr(ctx_len), k_cache.shape[1],
+                                               n, Hq, Hkv, hd, _lib.ptr(out), out.stride(0), _lib.ptr(ws),
+                                               k_cache.shape[0], _lib.ptr(_lib.status_word(q.device)), _lib.stream_ptr()),
+                  "paged_decode_even")
     return out
 
 
