@@ -15,6 +15,7 @@ __host__ __device__ inline bool epi_is_glu(int e) { return e == EPI_SWIGLU || e 
 // run concurrently share a band of the activation matrix that stays L2-resident and a handful of weight (B) tiles.
 struct SchedMFast {
   int m_tiles, n_tiles, group_m;
+  int early = 0;
   __device__ int tiles_for_cta(int cta, int ncta) const {
     const int total = m_tiles * n_tiles;
     return cta < total ? (total - cta + ncta - 1) / ncta : 0;
@@ -39,6 +40,7 @@ inline int pick_group_m(int m_tiles, int tile_rows, int K) {
 // covers kb_per K blocks of the main operand, the extra-K operand goes with split 0.
 struct SchedSplitK {
   int m_tiles, n_tiles, splits, kb_per, kb_main;
+  int early = 0;
   __device__ int tiles_for_cta(int cta, int ncta) const {
     const int total = m_tiles * n_tiles * splits;
     return cta < total ? (total - cta + ncta - 1) / ncta : 0;

@@ -118,6 +118,17 @@ struct NoComm {
   __device__ void finish(int* /*status*/) const {}
 };
 
+// Schedules with a member `early` set: B (and B2) are weights that no kernel still running writes, and the loads of the
+// first tile's first stages are issued before the wait for the previous kernel (see pdl_switch in host_utils.h).
+template <class S>
+__device__ __forceinline__ auto sched_early(const S& s, int) -> decltype(s.early) {
+  return s.early;
+}
+template <class S>
+__device__ __forceinline__ int sched_early(const S&, long) {
+  return 0;
+}
+
 // Optional epilogue hook `flush(row)`: called by every epilogue thread after its last tile (policies that defer work,
 // e.g. the publication of arrival flags, finish it there).
 template <class E>
@@ -175,8 +186,22 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_base_slot;
-  pdl_wait();                  // everything above overlapped the previous kernel's tail (when launched that way)
+  uint32_t early = 0;          // stages whose B tile is on its way already
+  if (threadIdx.x == 0 && my_tiles > 0 && sched_early(sched, 0)) {
+    const TileInfo ti = sched.get(blockIdx.x, gridDim.x, 0);
+    const int nmain = ti.kb_n < 0 ? kb_main : ti.kb_n;
+    early = min(STAGES, nmain + (ti.extra ? kb_extra : 0));
+    for (int s = 0; s < static_cast<int>(early); ++s) {
+      uint8_t* sb = smem + s * L::STAGE_BYTES + L::A_BYTES;
+      mbar_expect_tx(&full_bar[s], L::STAGE_BYTES);
+      if (s < nmain)
+        tma_load_2d(sb, &tmB, (ti.kb_lo + s) * GEMM_BK, ti.n_blk * BN + ti.b_row, &full_bar[s]);
+      else
+        tma_load_2d(sb, &tmB2, (s - nmain) * GEMM_BK, ti.n_blk * BN + ti.b_row, &full_bar[s]);
+    }
+  }
   pdl_launch_dependents();
+  pdl_wait();                  // everything above overlapped the previous kernel's tail (when launched that way)
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
@@ -207,14 +232,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           }
           uint8_t* sa = smem + s * L::STAGE_BYTES;
           uint8_t* sb = sa + L::A_BYTES;
-          mbar_expect_tx(&full_bar[s], L::STAGE_BYTES);
+          const bool b_due = it >= early;
+          if (b_due) mbar_expect_tx(&full_bar[s], L::STAGE_BYTES);
           if (kb < nmain) {
             tma_load_2d(sa, &tmA, (ti.kb_lo + kb) * GEMM_BK, ti.m_blk * GEMM_BM, &full_bar[s]);
-            tma_load_2d(sb, &tmB, (ti.kb_lo + kb) * GEMM_BK, ti.n_blk * BN + ti.b_row, &full_bar[s]);
+            if (b_due) tma_load_2d(sb, &tmB, (ti.kb_lo + kb) * GEMM_BK, ti.n_blk * BN + ti.b_row, &full_bar[s]);
           } else {
             const int k2 = (kb - nmain) * GEMM_BK;
             tma_load_2d(sa, &tmA2, k2, ti.m_blk * GEMM_BM, &full_bar[s]);
-            tma_load_2d(sb, &tmB2, k2, ti.n_blk * BN + ti.b_row, &full_bar[s]);
+            if (b_due) tma_load_2d(sb, &tmB2, k2, ti.n_blk * BN + ti.b_row, &full_bar[s]);
           }
         }
       }

@@ -39,6 +39,7 @@ struct Gemm2SmemLayout {
 // extra-K operands in that mode).
 struct SchedPair {
   int m_tiles2, n_tiles, group_m, splits, kb_per, kb_main;
+  int early = 0;
   __device__ int tiles_for_cta(int cluster, int nclusters) const {
     const int total = m_tiles2 * n_tiles * splits;
     return cluster < total ? (total - cluster + nclusters - 1) / nclusters : 0;
@@ -120,8 +121,24 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   cluster_wait();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_base_slot;
-  pdl_wait();                  // everything above overlapped the previous kernel's tail (when launched that way)
+  uint32_t early = 0;          // stages whose B tile is on its way already
+  if (threadIdx.x == 0 && my_tiles > 0 && sched_early(sched, 0)) {
+    const TileInfo ti = sched.get(cluster_id, n_clusters, 0);
+    const int row_b = ti.n_blk * G2_BN + static_cast<int>(rank) * G2_BNH + ti.b_row;
+    const int nmain = ti.kb_n < 0 ? kb_main : ti.kb_n;
+    early = min(STAGES, nmain + (ti.extra ? kb_extra : 0));
+    for (int s = 0; s < static_cast<int>(early); ++s) {
+      uint8_t* sb = smem + s * G2_STAGE_BYTES + L::A_BYTES;
+      if (leader) mbar_expect_tx(&full_bar[s], 2 * G2_STAGE_BYTES);
+      const uint32_t fb = mapa_shared(smem_u32(&full_bar[s]), 0);
+      if (s < nmain)
+        tma_load_2d_2cta(sb, &tmB, (ti.kb_lo + s) * GEMM_BK, row_b, fb);
+      else
+        tma_load_2d_2cta(sb, &tmB2, (s - nmain) * GEMM_BK, row_b, fb);
+    }
+  }
   pdl_launch_dependents();
+  pdl_wait();                  // everything above overlapped the previous kernel's tail (when launched that way)
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer (both CTAs)
@@ -157,15 +174,16 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           }
           uint8_t* sa = smem + s * G2_STAGE_BYTES;
           uint8_t* sb = sa + L::A_BYTES;
-          if (leader) mbar_expect_tx(&full_bar[s], 2 * G2_STAGE_BYTES);
+          const bool b_due = it >= early;
+          if (leader && b_due) mbar_expect_tx(&full_bar[s], 2 * G2_STAGE_BYTES);
           const uint32_t fb = mapa_shared(smem_u32(&full_bar[s]), 0);
           if (kb < nmain) {
             tma_load_2d_2cta(sa, &tmA, (ti.kb_lo + kb) * GEMM_BK, row_a, fb);
-            tma_load_2d_2cta(sb, &tmB, (ti.kb_lo + kb) * GEMM_BK, row_b, fb);
+            if (b_due) tma_load_2d_2cta(sb, &tmB, (ti.kb_lo + kb) * GEMM_BK, row_b, fb);
           } else {
             const int k2 = (kb - nmain) * GEMM_BK;
             tma_load_2d_2cta(sa, &tmA2, k2, row_a, fb);
-            tma_load_2d_2cta(sb, &tmB2, k2, row_b, fb);
+            if (b_due) tma_load_2d_2cta(sb, &tmB2, k2, row_b, fb);
           }
         }
       }

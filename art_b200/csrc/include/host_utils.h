@@ -62,10 +62,15 @@ inline int make_tmap_bf16_2d(CUtensorMap* out, const void* ptr, uint64_t rows, u
 // only its prologue (barrier / TMEM setup, descriptor prefetch, block scheduling) overlaps the predecessor's tail.  A
 // decode step is ~230 short launches whose hand-over gaps add up to a fifth of the step.  Kernels launched without
 // the attribute (everything while the switch is off, and all library kernels) keep full stream order.
+//
+// 2: the second operand of every product launched from now on (a projection's weights, adapter slots included) was
+// written by nothing that could still run, so the product's first weight tiles are requested before the wait.  A decode
+// step alternates products, which stream weights, with short kernels, which leave the memory idle.
 inline int& pdl_switch() {
   static int on = 0;
   return on;
 }
+inline int weights_early() { return pdl_switch() == 2; }
 
 template <class... KArgs, class... Args>
 inline cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

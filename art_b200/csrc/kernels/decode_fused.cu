@@ -145,8 +145,8 @@ decode_finalize_norm_kernel(float* __restrict__ ws, int ldw, int N, int kpad, co
                             __nv_bfloat16* __restrict__ h_out, int ldh) {
   __shared__ float t_s[DF_MAX_COLS];
   __shared__ float red[DF_THREADS / 32];
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.x;
   float* wrow = ws + static_cast<size_t>(row) * ldw;
   const int a = stage_shrink(wrow, N, kpad, cols, adapter, row, t_s);
@@ -213,7 +213,7 @@ decode_finalize_qkv_kernel(float* __restrict__ ws, int ldw, int Hq, int Hkv, int
                            long num_slots, int* status) {
   __shared__ float t_s[DF_MAX_COLS];
   __shared__ float cs_s[128], sn_s[128];     // cos / sin of the row's position for every frequency: shared by all heads
-  pdl_wait();
+  pdl_wait();                  // attention comes next: its first CTAs would share the few SMs that a product leaves free
   pdl_launch_dependents();
   const int row = blockIdx.x;
   const int q_size = Hq * hd, kv_size = Hkv * hd, N = q_size + 2 * kv_size;
@@ -314,9 +314,9 @@ ARTB_EXPORT int artb_decode_finalize_qkv(float* ws, int ldw, int M, int Hq, int 
 }
 
 // Programmatic dependent launch for the kernels of the decode step (see pdl_switch in host_utils.h); returns the
-// previous setting.  The engine turns it on around its decode body and off again afterwards.
+// previous setting.  The engine turns it on around its decode body and off again afterwards.  2: weights may be read early.
 ARTB_EXPORT int artb_set_pdl(int on) {
   const int prev = pdl_switch();
-  pdl_switch() = on ? 1 : 0;
+  pdl_switch() = on == 2 ? 2 : on != 0;
   return prev;
 }

@@ -33,6 +33,7 @@ static int launch_splitk(const CUtensorMap& tA, const CUtensorMap& tB, int kb_ma
   sched.splits = splits;
   sched.kb_per = (kb_main + splits - 1) / splits;
   sched.kb_main = kb_main;
+  sched.early = weights_early();
   int grid = sched.m_tiles * sched.n_tiles * splits;
   if (grid > sm_count()) grid = sm_count();
   EpiAtomic<BN> epi{ws, ldw, M, N};
@@ -48,8 +49,8 @@ __global__ void splitk_finalize_kernel(float* __restrict__ ws, int ldw, __nv_bfl
                                        const __nv_bfloat16* __restrict__ R, int ldr, int res_cols,
                                        const float* __restrict__ bias, int M, int N, const int* __restrict__ adapter,
                                        int mask_col0, int cols) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const int vec = N >> 2;
   const long total = static_cast<long>(M) * vec;
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < total;

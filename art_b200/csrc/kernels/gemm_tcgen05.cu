@@ -36,7 +36,7 @@ static int launch_gemm(const CUtensorMap& tA, const CUtensorMap& tB, const CUten
     configured[dev & 63] = true;
   }
   const int m_tiles = (M + GEMM_BM - 1) / GEMM_BM;
-  SchedMFast sched{m_tiles, (N + BN - 1) / BN, pick_group_m(m_tiles, GEMM_BM, kb_main * GEMM_BK)};
+  SchedMFast sched{m_tiles, (N + BN - 1) / BN, pick_group_m(m_tiles, GEMM_BM, kb_main * GEMM_BK), weights_early()};
   int grid = sched.m_tiles * sched.n_tiles;
   int cap = sm_count();
   if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
@@ -52,7 +52,7 @@ using namespace artb;
 // Tile width for an [M, N] output on `ctas` persistent CTAs: the widest tile that still fills the
 // machine.  Narrower tiles that would waste less of the last wave (224 for N = 3584: 6.92 waves
 // instead of 6.05) were measured and are no faster on a power-capped B200 (SMs idle in the last
-// wave let the others clock higher), so 224 / 192 are only used on request.
+// wave let the others clock higher), so 224 / 192 / 160 are only used on request (weight-streaming products of few rows).
 ARTB_EXPORT int artb_pick_bn(int M, int N, int ctas) {
   const long m_tiles = (M + GEMM_BM - 1) / GEMM_BM;
   if (N >= 256 && m_tiles * ((N + 255) / 256) >= ctas) return 256;
@@ -66,7 +66,7 @@ ARTB_EXPORT int artb_pick_bn(int M, int N, int ctas) {
 //   epilogue     : GemmEpilogue (EPI_SWIGLU_BWD: H = forward gate|up [M,2N] input, C = d(gate|up) [M,2N] output); R (bf16 [M,res_cols]) is added for EPI_BF16_RESID and, when given, for EPI_SWIGLU;
 //                  H (bf16 [M,N/2]) receives silu(gate)*up for EPI_SWIGLU, relu(gate)*up for EPI_RELUGLU (C may then be null);  res_cols 0 = all N columns; EPI_SILU, EPI_RELU2: their columns
 //   bias         : optional fp32 [N], added to the accumulator before any other epilogue step
-//   bn           : tile width 64 / 128 / 192 / 224 / 256 (0 = choose, see artb_pick_bn)
+//   bn           : tile width 64 / 128 / 160 / 192 / 224 / 256 (0 = choose, see artb_pick_bn)
 //   status       : device int32, receives a KernelStatus on a bounded-wait expiry (0 otherwise)
 //   max_ctas     : cap on the persistent grid (0 = one CTA per SM)
 // Returns 0, a negative HostError, or a positive cudaError_t.
@@ -87,7 +87,7 @@ ARTB_EXPORT int artb_gemm_bf16_tn(const void* A, int lda, const void* B, int ldb
   if ((epi_is_glu(epilogue) || epilogue == EPI_SWIGLU_BWD) && (!H || (ldh & 7) || (N & 31) || (reinterpret_cast<uintptr_t>(H) & 15)))
     return ERR_BAD_ALIGN;
   if (bn == 0) bn = artb_pick_bn(M, N, max_ctas > 0 && max_ctas < sm_count() ? max_ctas : sm_count());
-  if (bn != 64 && bn != 128 && bn != 192 && bn != 224 && bn != 256) return ERR_BAD_SHAPE;
+  if (bn != 64 && bn != 128 && bn != 160 && bn != 192 && bn != 224 && bn != 256) return ERR_BAD_SHAPE;
 
   CUtensorMap tA, tB, tA2, tB2;
   int e;
@@ -117,6 +117,7 @@ ARTB_EXPORT int artb_gemm_bf16_tn(const void* A, int lda, const void* B, int ldb
   if (bn == 256) ARTB_LAUNCH(256, 4)
   if (bn == 224) ARTB_LAUNCH(224, 4)
   if (bn == 192) ARTB_LAUNCH(192, 4)
+  if (bn == 160) ARTB_LAUNCH(160, 5)
   if (bn == 128) ARTB_LAUNCH(128, 6)
   ARTB_LAUNCH(64, 8)
 #undef ARTB_LAUNCH

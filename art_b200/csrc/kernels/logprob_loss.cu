@@ -59,6 +59,7 @@ struct SchedVocabSplit {
 // of 256 where the mean is 4.0.
 struct SchedVocabSpan {
   int m_tiles, n_tiles, splits;
+  int early = 0;
   __device__ int lo(int s) const { return static_cast<int>(static_cast<long>(s) * n_tiles / splits); }
   __device__ int tiles_for_cta(int cta, int) const {
     const int s = cta / m_tiles;
@@ -637,7 +638,7 @@ static int launch_sample(const void* H, int ldh, const void* W, int ldw, const S
     if (ce != cudaSuccess) return static_cast<int>(ce);
     configured[dev & 63] = true;
   }
-  const SchedVocabSpan sched{p.m_tiles, p.n_tiles, p.splits};
+  const SchedVocabSpan sched{p.m_tiles, p.n_tiles, p.splits, weights_early()};
   return static_cast<int>(launch_kernel(kern, dim3(p.m_tiles * p.splits), dim3(gemm_pipe_threads<EpiSample<BN>>()), L::TOTAL,
                                         stream, tA, tB, tA, tB, (K + GEMM_BK - 1) / GEMM_BK, 0, sched, epi, status, NoComm{}));
 }

@@ -293,7 +293,7 @@ class EngineLinear:
 
     def __call__(self, x, adapter_ids, any_lora: bool, residual=None, swiglu_out=None):
         from ..ops import elementwise as ew
-        from ..ops.gemm import gemm_splitk_, gemm_tn, plan_small_m, splitk_finalize
+        from ..ops.gemm import gemm_splitk_, gemm_tn, plan_small_m, splitk_finalize, stream_bn
         from ..ops.paged import lora_slot_mask_
 
         M = x.shape[0]
@@ -319,7 +319,7 @@ class EngineLinear:
             # residual / SwiGLU epilogue runs in the weight-streaming GEMM itself (no [M, N] intermediate)
             T = self._shrink(x, adapter_ids)
             return gemm_tn(x, self.W, a2=T, b2=self.B_all, residual=residual, swiglu_out=swiglu_out, two_cta=pair,
-                           bias=None if self.bias_ext is None else self.bias_ext[:N])
+                           bn=0 if pair else stream_bn(M, N), bias=None if self.bias_ext is None else self.bias_ext[:N])
         Next = N + self.kpad if any_lora else N
         Wv = self.W_ext[:Next]
         bias = None if self.bias_ext is None else self.bias_ext[:Next]
@@ -334,8 +334,8 @@ class EngineLinear:
             # the finalize pass also applies the per-row adapter-slot mask to the shrink columns
             splitk_finalize(ws, y_ext, bias, residual, N, adapter_ids if any_lora else None, N, self.cols)
         else:
-            gemm_tn(x, Wv, out=y_ext, bias=bias, residual=residual, res_cols=N, bn=0 if pair else bn, two_cta=pair,
-                    swiglu_out=swiglu_out if fuse_swiglu else None)
+            gemm_tn(x, Wv, out=y_ext, bias=bias, residual=residual, res_cols=N, two_cta=pair,
+                    bn=0 if pair else stream_bn(M, Next) or bn, swiglu_out=swiglu_out if fuse_swiglu else None)
         if not any_lora:
             if swiglu_out is not None and not fuse_swiglu:
                 ew.swiglu_fwd(y_ext, out=swiglu_out)
@@ -517,7 +517,7 @@ class DeviceRunner:
     def _decode_body(self, st, n_steps: int, any_lora: bool, splits: int, ws, restricted: bool = False, procs=None):
         from ..ops import paged
 
-        prev_pdl = paged.set_pdl(self.overlap_launches and os.environ.get("ARTB_PDL", "1") != "0")
+        prev_pdl = paged.set_pdl(2 if self.overlap_launches and os.environ.get("ARTB_PDL", "1") != "0" else 0)
         try:
             self._decode_steps(st, n_steps, any_lora, splits, ws, restricted, procs)
         finally:

@@ -218,10 +218,24 @@ def plan_small_m(M: int, N: int, K: int, sms: int = 148, pair: bool = False) -> 
     m_tiles = (M + 127) // 128
     bn = 256 if N >= 256 else (128 if N >= 128 else 64)
     tiles = m_tiles * ((N + bn - 1) // bn)
-    if tiles >= 100:
-        return bn, 1
-    splits = max(1, min(sms // tiles, max(1, kb // 4)))
+    most = max(1, kb // 4)
+    splits = max(1, min(sms // tiles, most))
+    if bn == 256 and 3 * tiles * splits < 2 * sms and splits > 1:
+        # a short K does not give enough slices: narrower tiles do (2048 x 2048 weights: 128 CTAs instead of 64)
+        tiles = m_tiles * ((N + 127) // 128)
+        return 128, max(1, min(sms // tiles, most))
     return bn, splits
+
+
+def stream_bn(M: int, N: int, sms: int = 148) -> int:
+    """Tile width of an unsplit weight-streaming GEMM of up to 256 rows: the one whose busiest CTA streams the fewest
+    weight rows, the widest where they tie.  22016 x 2048 weights are 86 tiles of 256 or 138 of 160; 24576 x 4096 are 192
+    of 128, in two waves (51 us for 64 rows), or 128 of 192 (42 us).  More rows are bound by arithmetic: 0, for the choice
+    of the product itself."""
+    if M > 256 or N < 256:
+        return 0
+    m_tiles = (M + 127) // 128
+    return min((256, 224, 192, 160, 128), key=lambda w: (-(-(m_tiles * -(-N // w)) // sms) * w, -w))
 
 
 _skinny_ws: dict = {}

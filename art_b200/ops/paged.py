@@ -54,11 +54,12 @@ def kv_write(qkv: torch.Tensor, k_col: int, v_col: int, slot: torch.Tensor, k_ca
                                       _lib.ptr(_lib.status_word(qkv.device)), _lib.stream_ptr()), "kv_write")
 
 
-def set_pdl(on: bool) -> bool:
+def set_pdl(on: bool | int) -> int:
     """Programmatic dependent launch for the decode-step kernels launched from now on (returns the previous setting):
     each may start its prologue while its predecessor in the stream drains, and waits on the device before touching
-    global memory."""
-    return bool(_f("artb_set_pdl")(1 if on else 0))
+    global memory.  ``2``: products may also request their second operand (weights that no kernel in flight writes) before
+    the wait."""
+    return _f("artb_set_pdl")(int(on))
 
 
 def decode_finalize_norm(ws: torch.Tensor, M: int, N: int, kpad: int, x_out: torch.Tensor, *, bias: torch.Tensor | None = None,
