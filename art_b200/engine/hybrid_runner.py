@@ -85,9 +85,6 @@ def kernel_sources(cfg: HybridConfig) -> set[str]:
 
 class HybridRunner(DeviceRunner):
     mixed_steps = True
-    # One-CTA and CTA-pair products follow one another directly here (per-head products in front of an output projection);
-    # with overlapping launches their tensor-memory allocations would meet on an SM.  Full stream order between kernels.
-    overlap_launches = False
 
     def __init__(self, cfg: HybridConfig, kv, base: dict[str, torch.Tensor], *, device="cuda", dtype: torch.dtype = torch.bfloat16,
                  max_loras: int = 0):
@@ -721,6 +718,12 @@ class HybridRunner(DeviceRunner):
 
     def _stage_sequences(self, st, seqs, nb: int) -> None:
         st["state_slot"].copy_(torch.tensor([s.state_slot for s in seqs] + [-1] * (nb - len(seqs)), dtype=torch.int32), non_blocking=True)
+
+    def _overlap(self, nb: int) -> bool:
+        # One-CTA and CTA-pair products follow one another directly here (per-head products in front of an output
+        # projection); with overlapping launches their tensor-memory allocations would meet on an SM.  Pairs serve batches
+        # of whole 256 rows, which keep full stream order between kernels.
+        return nb % 256 != 0
 
     def _attn_splits(self, nb: int, max_ctx: int) -> int:
         """Stands for how far the batch's tokens reach back (a power of two): the attention layers plan their splits by it.

@@ -514,10 +514,13 @@ class DeviceRunner:
             self._dstate[key] = st
         return st
 
+    def _overlap(self, nb: int) -> bool:
+        return self.overlap_launches
+
     def _decode_body(self, st, n_steps: int, any_lora: bool, splits: int, ws, restricted: bool = False, procs=None):
         from ..ops import paged
 
-        prev_pdl = paged.set_pdl(2 if self.overlap_launches and os.environ.get("ARTB_PDL", "1") != "0" else 0)
+        prev_pdl = paged.set_pdl(2 if self._overlap(st["tokens"].shape[0]) and os.environ.get("ARTB_PDL", "1") != "0" else 0)
         try:
             self._decode_steps(st, n_steps, any_lora, splits, ws, restricted, procs)
         finally:
