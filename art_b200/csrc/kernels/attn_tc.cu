@@ -47,8 +47,10 @@ struct TcSmem {
   static constexpr int GK = P + TC_TILE;           // int [8 warps][64]: key group ids of a partially masked tile
   static constexpr int XCH = GK + 8 * 64 * 4;      // float [2][2][128]: row max / row sum exchange between warp pairs
   static constexpr int BAR = XCH + 2 * 256 * 4;    // 21 mbarriers + tmem slot + abort
-  static constexpr int TOTAL = BAR + 28 * 8 + 1024;
+  static constexpr int LIST = BAR + 28 * 8;        // uint16 [S / 128]: the key tiles to visit
+  static constexpr int TOTAL = LIST + 1024;        // + the list
 };
+constexpr int TC_MAX_TILES = 8192;                 // of a row: what the list may take of the shared memory
 
 // k-step kk (16 elements) of a [128 x 128] K-major tile stored as two 64-column halves
 __device__ __forceinline__ uint64_t tc_desc(uint32_t tile_base, int kk) {
@@ -58,16 +60,16 @@ __device__ __forceinline__ uint64_t tc_desc(uint32_t tile_base, int kk) {
 __device__ __forceinline__ int tc_state128(const uint8_t* st64, int nb64, int qb, int kb) {
   const uint8_t* r0 = st64 + static_cast<size_t>(2 * qb) * nb64 + 2 * kb;
   const uint8_t* r1 = r0 + nb64;
-  const int a = r0[0], b = r0[1], c = r1[0], d = r1[1];
-  if ((a | b | c | d) == 0) return 0;
-  return (a == 2 && b == 2 && c == 2 && d == 2) ? 2 : 1;
+  const int a = *reinterpret_cast<const uint16_t*>(r0), b = *reinterpret_cast<const uint16_t*>(r1);    // nb64 is even
+  if ((a | b) == 0) return 0;
+  return (a == 0x0202 && b == 0x0202) ? 2 : 1;
 }
 
 __global__ void __launch_bounds__(TC_THREADS, 1)
 attn_tc_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_constant__ CUtensorMap tmVt,
                    const int* __restrict__ gid, const int* __restrict__ pid, const uint8_t* __restrict__ state,
                    __nv_bfloat16* __restrict__ out, int ldo, float* __restrict__ lse2, int S, int Hq, int Hkv,
-                   float scale_log2, long M, int* status) {
+                   float scale_log2, long M, const uint8_t* __restrict__ wanted, int* status) {
   extern __shared__ uint8_t tc_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tc_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + TcSmem::BAR);
@@ -90,10 +92,13 @@ attn_tc_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
   const int nb = S / TC_B, nb64 = S / 64;
   const int qb = nb - 1 - blockIdx.x;      // heavy (late) query tiles first
   const int h = blockIdx.y, row = blockIdx.z;
+  if (wanted && !wanted[row * nb + qb]) return;      // the whole CTA
   const int kvh = h / (Hq / Hkv);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long base = static_cast<long>(row) * S;
   const uint8_t* st64 = state + static_cast<size_t>(row) * nb64 * nb64;
+  uint16_t* list = reinterpret_cast<uint16_t*>(smem + TcSmem::LIST);
+  __shared__ int s_found[TC_THREADS / 32];
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
@@ -116,6 +121,24 @@ attn_tc_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  // The key tiles that are not fully masked, in order, as 2 * tile + (partly masked).  Every role used to walk the table by
+  // itself, a dependent load per tile: with 24 prompts side by side a CTA visits 3 of up to 116 tiles and the walk was
+  // most of its 41 us.
+  int n_tiles = 0;
+  for (int kb0 = 0; kb0 <= qb; kb0 += TC_THREADS) {
+    const int kb = kb0 + static_cast<int>(threadIdx.x);
+    const int st = kb <= qb ? tc_state128(st64, nb64, qb, kb) : 0;
+    const uint32_t hit = __ballot_sync(0xffffffffu, st != 0);
+    if (lane == 0) s_found[warp] = __popc(hit);
+    __syncthreads();
+    int at = n_tiles;
+    for (int w = 0; w < TC_THREADS / 32; ++w) {
+      if (w < warp) at += s_found[w];
+      n_tiles += s_found[w];
+    }
+    if (st != 0) list[at + __popc(hit & ((1u << lane) - 1u))] = static_cast<uint16_t>(2 * kb + (st == 1));
+    __syncthreads();
+  }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -130,9 +153,8 @@ attn_tc_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
       const int qrow = static_cast<int>(base) + qb * TC_B;
       tma_load_2d(smem + TcSmem::Q, &tmQK, h * TC_HD, qrow, q_full);
       tma_load_2d(smem + TcSmem::Q + TC_HALF, &tmQK, h * TC_HD + 64, qrow, q_full);
-      uint32_t it = 0;
-      for (int kb = 0; kb <= qb && !*abort_flag; ++kb) {
-        if (tc_state128(st64, nb64, qb, kb) == 0) continue;
+      for (int it = 0; it < n_tiles && !*abort_flag; ++it) {
+        const int kb = list[it] >> 1;
         const int s = it & 1;
         if (!mbar_wait(&kv_empty[s], ((it >> 1) & 1) ^ 1)) {
           atomicMax(status, ST_TIMEOUT_EMPTY);
@@ -148,7 +170,6 @@ attn_tc_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
         mbar_expect_tx(&v_full[s], TC_TILE);
         tma_load_2d(sv, &tmVt, krow, kvh * TC_HD, &v_full[s]);
         tma_load_2d(sv + TC_HALF, &tmVt, krow + 64, kvh * TC_HD, &v_full[s]);
-        ++it;
       }
     }
   } else if (warp == 1) {
@@ -176,8 +197,7 @@ attn_tc_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
         return true;
       };
       uint32_t it = 0;
-      for (int kb = 0; kb <= qb && ok && !*abort_flag; ++kb) {
-        if (tc_state128(st64, nb64, qb, kb) == 0) continue;
+      for (int i = 0; i < n_tiles && ok && !*abort_flag; ++i) {
         const int s = it & 1;
         const uint32_t ph = (it >> 1) & 1;
         if (!mbar_wait(&k_full[s], ph) || !mbar_wait(&s_empty[s], ph ^ 1)) {
@@ -263,15 +283,14 @@ attn_tc_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
       return true;
     };
 
-    for (int kb = 0; kb <= qb; ++kb) {
-      const int stt = tc_state128(st64, nb64, qb, kb);
-      if (stt == 0) continue;
+    for (int i = 0; i < n_tiles; ++i) {
+      const int kb = list[i] >> 1;
       if (__shfl_sync(0xffffffffu, *abort_flag, 0)) {
         dead = true;
         break;
       }
       const int s = it & 1;
-      const bool partial = stt == 1;
+      const bool partial = list[i] & 1;
       if (partial) {
         __syncwarp();
         gk[lane] = gid[base + kb * TC_B + hf * 64 + lane];
@@ -413,10 +432,12 @@ __global__ void attn_tc_transpose_v_kernel(const __nv_bfloat16* __restrict__ qkv
 using namespace artb;
 
 // qkv [rows*S, ld] post-RoPE, head dim 128, S % 128 == 0; vt: scratch bf16 [Hkv*128, rows*S]; state: the
-// 64 x 64 tile-state table of artb_attn_tile_states; out [rows*S, Hq*128]; lse2 [Hq, rows*S].
+// 64 x 64 tile-state table of artb_attn_tile_states; wanted: uint8 [rows, S / 128], null for all: the query tiles to
+// compute, rows of the others are left as they are; out [rows*S, Hq*128]; lse2 [Hq, rows*S].
 ARTB_EXPORT int artb_attn_tc_fwd(const void* qkv, int ld, const int* gid, const int* pid, const uint8_t* state,
                                  void* vt, void* out, int ldo, float* lse2, int rows, int S, int Hq, int Hkv,
-                                 int* status, cudaStream_t st) {
+                                 const uint8_t* wanted, int* status, cudaStream_t st) {
+  if (S / TC_B > TC_MAX_TILES) return ERR_TOO_LARGE;
   if (S % TC_B || Hq % Hkv || (ld & 7) || (ldo & 7)) return ERR_BAD_SHAPE;
   const long M = static_cast<long>(rows) * S;
   if (M > 0x7fffffffL || (M & 7)) return ERR_BAD_SHAPE;
@@ -434,14 +455,15 @@ ARTB_EXPORT int artb_attn_tc_fwd(const void* qkv, int ld, const int* gid, const 
   int dev = 0;
   cudaGetDevice(&dev);
   if (!configured[dev & 63]) {
-    cudaError_t ce = cudaFuncSetAttribute(attn_tc_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TcSmem::TOTAL);
+    cudaError_t ce = cudaFuncSetAttribute(attn_tc_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          TcSmem::TOTAL + 2 * TC_MAX_TILES);
     if (ce != cudaSuccess) return static_cast<int>(ce);
     configured[dev & 63] = true;
   }
   const float scale_log2 = 1.4426950408889634f / sqrtf(static_cast<float>(TC_HD));
   dim3 grid(S / TC_B, Hq, rows);
-  attn_tc_fwd_kernel<<<grid, TC_THREADS, TcSmem::TOTAL, st>>>(tmQK, tmVt, gid, pid, state,
+  attn_tc_fwd_kernel<<<grid, TC_THREADS, TcSmem::TOTAL + 2 * (S / TC_B), st>>>(tmQK, tmVt, gid, pid, state,
                                                               reinterpret_cast<__nv_bfloat16*>(out), ldo, lse2, S, Hq,
-                                                              Hkv, scale_log2, M, status);
+                                                              Hkv, scale_log2, M, wanted, status);
   return static_cast<int>(cudaGetLastError());
 }

@@ -291,7 +291,8 @@ class EngineLinear:
             return splitk_finalize(ws, T, None, None, 0, adapter_ids, 0, self.cols)
         return lora_slot_mask_(gemm_tn(x, self.A_all, bn=bn), adapter_ids, self.cols)
 
-    def __call__(self, x, adapter_ids, any_lora: bool, residual=None, swiglu_out=None):
+    def __call__(self, x, adapter_ids, any_lora: bool, residual=None, swiglu_out=None, out=None):
+        """``out``: where the product of more than 512 rows goes."""
         from ..ops import elementwise as ew
         from ..ops.gemm import gemm_splitk_, gemm_tn, plan_small_m, splitk_finalize, stream_bn
         from ..ops.paged import lora_slot_mask_
@@ -301,9 +302,9 @@ class EngineLinear:
             if any_lora:
                 T = gemm_tn(x, self.A_all, bn=64)
                 lora_slot_mask_(T, adapter_ids, self.cols)
-                return gemm_tn(x, self.W, a2=T, b2=self.B_all, residual=residual, swiglu_out=swiglu_out,
+                return gemm_tn(x, self.W, a2=T, b2=self.B_all, residual=residual, swiglu_out=swiglu_out, out=out,
                                bias=None if self.bias_ext is None else self.bias_ext[:self.N])
-            return gemm_tn(x, self.W, residual=residual, swiglu_out=swiglu_out,
+            return gemm_tn(x, self.W, residual=residual, swiglu_out=swiglu_out, out=out,
                            bias=None if self.bias_ext is None else self.bias_ext[:self.N])
         N = self.N
         if _DECODE_PLAN == "narrow" and self.K <= NARROW_MAX_K and swiglu_out is None and 128 <= M <= 512:
@@ -809,12 +810,12 @@ class NativeRunner(DeviceRunner):
         L["gu"](h2, adapter_ids, any_lora, swiglu_out=hact)
         return self._reduce(L["down"](hact, adapter_ids, any_lora, residual=self._res(x2)))
 
-    def _qkv(self, L, x, pos, adapter_ids, any_lora):
+    def _qkv(self, L, x, pos, adapter_ids, any_lora, out=None):
         from ..ops import elementwise as ew
 
         cfg = self.cfg
         h1, _ = ew.rmsnorm_fwd(x, L["ln1"], cfg.rms_norm_eps, want_rstd=False)
-        qkv = L["qkv"](h1, adapter_ids, any_lora)
+        qkv = L["qkv"](h1, adapter_ids, any_lora, out=out)
         if cfg.qk_norm:
             ew.headnorm_fwd_(qkv, L["q_norm"], 0, cfg.num_heads, cfg.head_dim, cfg.rms_norm_eps)
             ew.headnorm_fwd_(qkv, L["k_norm"], cfg.q_size, cfg.num_kv_heads, cfg.head_dim, cfg.rms_norm_eps)
@@ -853,11 +854,12 @@ class NativeRunner(DeviceRunner):
             row_ranges.append((r0, len(tok)))
             last_rows.append(len(tok) - 1)
         M = len(tok)
-        S_att = (att + 63) // 64 * 64
+        Hq, Hkv, hd = cfg.num_heads, cfg.num_kv_heads, cfg.head_dim
+        step = 128 if hd == 128 else 64         # the tensor-core attention of head dim 128 takes whole 128-query tiles
+        S_att = (att + step - 1) // step * step
         gid += [-(j + 1) for j in range(S_att - att)]
         any_lora = any(a >= 0 for a in adapter)
         self._moe_mixed = any_lora and any(a < 0 for a in adapter)
-        use_index = bool(cached_spans) or S_att != M
         t_tok = torch.tensor(tok, dtype=torch.int64, device=dev)
         t_pos = torch.tensor(pos, dtype=torch.int32, device=dev)
         t_ad = torch.tensor(adapter, dtype=torch.int32, device=dev)
@@ -865,21 +867,26 @@ class NativeRunner(DeviceRunner):
         t_gid = torch.tensor(gid, dtype=torch.int32, device=dev)
         t_rows = torch.tensor(new_rows, dtype=torch.int64, device=dev)
         plan = attn_ops.make_plan(t_gid, t_gid, S_att, "native")
-        Hq, Hkv, hd = cfg.num_heads, cfg.num_kv_heads, cfg.head_dim
+        if cached_spans and step == 128:        # tiles without a new token are not computed
+            plan.wanted = torch.zeros(S_att // step, dtype=torch.uint8, device=dev).index_fill_(0, t_rows // step, 1)
+        # the rows of attention: one buffer for all layers, each of which writes every row that a token has; without cached
+        # tokens the projection's rows are the buffer's first
+        buf = torch.empty((S_att, cfg.q_size + 2 * cfg.kv_size), dtype=self.embed.dtype, device=dev)
+        buf[att:].zero_()
+        place = not cached_spans and M > 512
         x = ew.gather_rows(self.embed, t_tok)
         span_tables = [(a0, nc, torch.tensor(bl, dtype=torch.int32, device=dev)) for a0, nc, bl in cached_spans]
         for li, L in enumerate(self.layers):
-            qkv = self._qkv(L, x, t_pos, t_ad, any_lora)
+            qkv = self._qkv(L, x, t_pos, t_ad, any_lora, out=buf[:M] if place else None)
             paged.kv_write(qkv, cfg.q_size, cfg.q_size + cfg.kv_size, t_slot, self.kv.k[li], self.kv.v[li])
-            if use_index:
-                buf = torch.zeros((S_att, qkv.shape[1]), dtype=qkv.dtype, device=dev)
-                buf.index_copy_(0, t_rows, qkv)
+            if cached_spans:
+                buf.index_copy_(0, t_rows, qkv[:, :buf.shape[1]])
                 for a0, nc, bt in span_tables:
                     paged.kv_gather(self.kv.k[li], self.kv.v[li], bt, bs, nc, buf[a0:], cfg.q_size, cfg.q_size + cfg.kv_size)
-                o_all, _ = attn_ops.forward(buf, Hq, Hkv, hd, plan, need_grad=False)
-                o = o_all.index_select(0, t_rows)
-            else:
-                o, _ = attn_ops.forward(qkv, Hq, Hkv, hd, plan, need_grad=False)
+            elif not place:
+                buf[:M].copy_(qkv[:, :buf.shape[1]])
+            o, _ = attn_ops.forward(buf, Hq, Hkv, hd, plan, need_grad=False)
+            o = o.index_select(0, t_rows) if cached_spans else o[:M]
             x2 = self._reduce(L["o"](o, t_ad, any_lora, residual=self._res(x)))
             x = self._mlp(L, x2, t_ad, any_lora)
         return x, row_ranges

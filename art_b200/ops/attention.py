@@ -28,6 +28,7 @@ class AttnPlan:
     S: int
     state: torch.Tensor | None = None   # native: uint8 tile states
     mask: torch.Tensor | None = None    # sdpa: dense bool mask [rows,1,S,S]
+    wanted: torch.Tensor | None = None  # native, forward only: uint8 [rows, S / 128], the 128-query tiles that are used
 
 
 @dataclass

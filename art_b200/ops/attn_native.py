@@ -14,7 +14,7 @@ _sigs = {
     "artb_attn_tile_states": [vp, vp, vp, ci, ci, vp],
     "artb_attn_tree_fwd": [vp, ci, vp, vp, vp, vp, ci, vp, ci, ci, ci, ci, ci, vp],
     "artb_attn_tree_bwd": [vp, ci, vp, vp, ci, vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, ci, ci, vp],
-    "artb_attn_tc_fwd": [vp, ci, vp, vp, vp, vp, vp, ci, vp, ci, ci, ci, ci, vp, vp],
+    "artb_attn_tc_fwd": [vp, ci, vp, vp, vp, vp, vp, ci, vp, ci, ci, ci, ci, vp, vp, vp],
     "artb_attn_tc_bwd": [vp, ci, vp, vp, ci, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, ci, ci, ci, vp, vp],
     "artb_attn_tc_bwd_splits": [ci, ci, ci, ci],
 }
@@ -49,11 +49,11 @@ def forward(qkv: torch.Tensor, Hq: int, Hkv: int, hd: int, plan) -> tuple[torch.
     S = plan.S
     out = torch.empty((M, Hq * hd), dtype=qkv.dtype, device=qkv.device)
     lse2 = torch.empty((Hq, M), dtype=torch.float32, device=qkv.device)
-    if USE_TC and hd == 128 and S % 128 == 0 and M % 8 == 0:
+    if USE_TC and hd == 128 and S % 128 == 0 and M % 8 == 0 and S <= 1 << 20:
         vt = torch.empty((Hkv * hd, M), dtype=qkv.dtype, device=qkv.device)
         _lib.check_rc(_f("artb_attn_tc_fwd")(_lib.ptr(qkv), qkv.stride(0), _lib.ptr(plan.gid), _lib.ptr(plan.pid),
                                              _lib.ptr(plan.state), _lib.ptr(vt), _lib.ptr(out), out.stride(0),
-                                             _lib.ptr(lse2), M // S, S, Hq, Hkv,
+                                             _lib.ptr(lse2), M // S, S, Hq, Hkv, _lib.ptr(plan.wanted),
                                              _lib.ptr(_lib.status_word(qkv.device)), _lib.stream_ptr()), "attn_tc_fwd")
         return out, (qkv, out, lse2, Hq, Hkv, hd)
     _lib.check_rc(_f("artb_attn_tree_fwd")(_lib.ptr(qkv), qkv.stride(0), _lib.ptr(plan.gid), _lib.ptr(plan.pid),
