@@ -9,7 +9,8 @@
 //
 //   decode_finalize_norm   y = ws + bias + residual + T_slot (sB_slot)^T ;  x_out = bf16(y) ;  h_out = RMSNorm(x_out) w
 //                          (after the o and down projections; the norm is the next block's input norm)
-//   decode_finalize_qkv    q|k|v = ws + bias + T_slot (sB_slot)^T ;  RoPE on q and k ;  q -> q_out, k / v -> KV cache
+//   decode_finalize_qkv    q|k|v = ws + bias + T_slot (sB_slot)^T ;  RMSNorm of each q and k head where the model has it ;
+//                          RoPE on q and k ;  q -> q_out, k / v -> KV cache
 //
 // A row belongs to ONE adapter slot, so the LoRA expand is a dot product of `cols` (= modules x rank, 8..24) shrink
 // values with the row's slice of sB (kept transposed for this purpose, [shrink column, output feature]): CUDA-core
@@ -208,7 +209,8 @@ __global__ void __launch_bounds__(DQ_THREADS, 2)
 decode_finalize_qkv_kernel(float* __restrict__ ws, int ldw, int Hq, int Hkv, int hd, int kpad,
                            const float* __restrict__ bias, const int* __restrict__ adapter,
                            const __nv_bfloat16* __restrict__ B_all, int ldb, int cols, const int* __restrict__ pos,
-                           float log2_theta, const int* __restrict__ slot, __nv_bfloat16* __restrict__ k_cache,
+                           float log2_theta, const __nv_bfloat16* __restrict__ q_norm, const __nv_bfloat16* __restrict__ k_norm,
+                           float eps, const int* __restrict__ slot, __nv_bfloat16* __restrict__ k_cache,
                            __nv_bfloat16* __restrict__ v_cache, __nv_bfloat16* __restrict__ q_out, int ldq,
                            long num_slots, int* status) {
   __shared__ float t_s[DF_MAX_COLS];
@@ -240,6 +242,25 @@ decode_finalize_qkv_kernel(float* __restrict__ ws, int ldw, int Hq, int Hkv, int
         add_bias8(x2, bias + c2);
       }
       if (a >= 0) lora_expand8x2(x1, x2, t_s, Bs, ldb, c1, c2, cols);
+      if (q_norm) {
+        // a head's values lie in per_head (a power of two) neighbouring lanes: one pass instead of two kernels over
+        // q and k in memory, two more for the rotation and the cache write (12 us of a layer's 150 beside attention)
+        float ss = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) ss = fmaf(x1[e], x1[e], fmaf(x2[e], x2[e], ss));
+        const uint32_t group = per_head == 32 ? 0xffffffffu : ((1u << per_head) - 1u) << (threadIdx.x & 31 & ~(per_head - 1));
+        for (int o = per_head >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(group, ss, o);
+        const float r = rsqrtf(ss / hd + eps);
+        const __nv_bfloat16* nw = (h < Hq ? q_norm : k_norm) + vv * 8;
+        float w1[8], w2[8];
+        ld8(nw, w1);
+        ld8(nw + half, w2);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          x1[e] *= r * w1[e];
+          x2[e] *= r * w2[e];
+        }
+      }
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const float sn = sn_s[vv * 8 + e], cs = cs_s[vv * 8 + e];
@@ -297,18 +318,22 @@ ARTB_EXPORT int artb_decode_finalize_norm(float* ws, int ldw, int M, int N, int 
 #undef ARTB_DF
 }
 
+// q_norm, k_norm (bf16 [hd], or both null): weights of the RMSNorm of each head, hd a power of two.
 // k_cache / v_cache: [slots, Hkv * hd] bf16 (slot = block * block_size + offset; slot[m] < 0: row not written).
 ARTB_EXPORT int artb_decode_finalize_qkv(float* ws, int ldw, int M, int Hq, int Hkv, int hd, int kpad, const float* bias,
                                          const int* adapter, const void* B_all, int ldb, int cols, const int* pos,
-                                         float theta, const int* slot, void* k_cache, void* v_cache, void* q_out, int ldq,
-                                         long num_slots, int* status, cudaStream_t st) {
+                                         float theta, const void* q_norm, const void* k_norm, float eps, const int* slot,
+                                         void* k_cache, void* v_cache, void* q_out, int ldq, long num_slots, int* status,
+                                         cudaStream_t st) {
   if (M <= 0) return 0;
   if ((hd & 15) || hd > 256 || (ldw & 3) || (ldq & 7) || Hq <= 0 || Hkv <= 0 || !pos || !slot) return ERR_BAD_SHAPE;
+  if (!q_norm != !k_norm || (q_norm && (hd & (hd - 1)))) return ERR_BAD_SHAPE;
   if (adapter && (cols <= 0 || cols > DF_MAX_COLS || (kpad & 3) || (ldb & 7) || !B_all)) return ERR_BAD_SHAPE;
   if (reinterpret_cast<uintptr_t>(ws) & 15) return ERR_BAD_ALIGN;
   return static_cast<int>(launch_kernel(
       decode_finalize_qkv_kernel, dim3(M), dim3(DQ_THREADS), 0, st, ws, ldw, Hq, Hkv, hd, kpad, bias, adapter,
-      reinterpret_cast<const __nv_bfloat16*>(B_all), ldb, cols, pos, log2f(theta), slot,
+      reinterpret_cast<const __nv_bfloat16*>(B_all), ldb, cols, pos, log2f(theta),
+      reinterpret_cast<const __nv_bfloat16*>(q_norm), reinterpret_cast<const __nv_bfloat16*>(k_norm), eps, slot,
       reinterpret_cast<__nv_bfloat16*>(k_cache), reinterpret_cast<__nv_bfloat16*>(v_cache),
       reinterpret_cast<__nv_bfloat16*>(q_out), ldq, num_slots, status));
 }

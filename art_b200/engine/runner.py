@@ -946,9 +946,10 @@ class NativeRunner(DeviceRunner):
 
     def _fused_decode_ok(self, M: int) -> bool:
         """The fused finish kernels cover one GPU per replica (a tensor-parallel replica all-reduces between the
-        projection and the norm), no per-head q/k norm, the unscaled rotary embedding, dense MLPs, and adapter slots
+        projection and the norm), per-head q/k norms of a power of two, the unscaled rotary embedding, dense MLPs, and adapter slots
         of at most 64 shrink columns."""
-        if (self.tp > 1 or self.cfg.qk_norm or self.cfg.rope_scaling is not None or M > 512
+        hd = self.cfg.head_dim
+        if (self.tp > 1 or (self.cfg.qk_norm and hd & (hd - 1)) or self.cfg.rope_scaling is not None or M > 512
                 or os.environ.get("ARTB_DECODE_FUSED", "1") == "0"):
             return False
         L = self.layers[0]
@@ -965,7 +966,8 @@ class NativeRunner(DeviceRunner):
         w = lin.partial_sums(h, any_lora)
         paged.decode_finalize_qkv(w, M, Hq, Hkv, hd, lin.kpad, st["pos"], cfg.rope_theta, st["slot"], self.kv.k[li],
                                   self.kv.v[li], st["q"], bias=None if lin.bias_ext is None else lin.bias_ext[:lin.N],
-                                  adapter=ad, B_all=lin.B_T, cols=lin.cols)
+                                  adapter=ad, B_all=lin.B_T, cols=lin.cols, q_norm=L["q_norm"] if cfg.qk_norm else None,
+                                  k_norm=L["k_norm"] if cfg.qk_norm else None, eps=cfg.rms_norm_eps)
         paged.paged_decode_even(st["q"], self.kv.k[li], self.kv.v[li], st["bt"], st["ctx"], Hq, Hkv, hd, st["attn_out"], st["attn_ws"])
         lin = L["o"]
         w = lin.partial_sums(st["attn_out"], any_lora)

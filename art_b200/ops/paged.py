@@ -25,8 +25,8 @@ _sigs = {
     "artb_top_logprobs": [vp, cl, vp, ci, ci, ci, vp, vp, vp],
     "artb_set_pdl": [ci],
     "artb_decode_finalize_norm": [vp, ci, ci, ci, ci, vp, vp, ci, vp, vp, ci, ci, vp, ctypes.c_float, vp, ci, vp, ci, vp],
-    "artb_decode_finalize_qkv": [vp, ci, ci, ci, ci, ci, ci, vp, vp, vp, ci, ci, vp, ctypes.c_float, vp, vp, vp, vp, ci, cl, vp,
-                                 vp],
+    "artb_decode_finalize_qkv": [vp, ci, ci, ci, ci, ci, ci, vp, vp, vp, ci, ci, vp, ctypes.c_float, vp, vp, ctypes.c_float, vp, vp,
+                                 vp, vp, ci, cl, vp, vp],
 }
 _bound: dict[str, object] = {}
 
@@ -80,12 +80,14 @@ def decode_finalize_norm(ws: torch.Tensor, M: int, N: int, kpad: int, x_out: tor
 def decode_finalize_qkv(ws: torch.Tensor, M: int, Hq: int, Hkv: int, hd: int, kpad: int, pos: torch.Tensor, theta: float,
                         slot: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, q_out: torch.Tensor, *,
                         bias: torch.Tensor | None = None, adapter: torch.Tensor | None = None,
-                        B_all: torch.Tensor | None = None, cols: int = 0) -> None:
+                        B_all: torch.Tensor | None = None, cols: int = 0, q_norm: torch.Tensor | None = None,
+                        k_norm: torch.Tensor | None = None, eps: float = 1e-6) -> None:
     """Finish the decode-time q|k|v projection from its split-K workspace: bias, LoRA expand of the row's adapter slot,
-    RoPE on q and k; q goes to ``q_out`` [M, Hq*hd], k and v straight into the paged cache at ``slot``."""
+    the RMSNorm of each head (``q_norm`` and ``k_norm``, for head dims that are powers of two), RoPE on q and k; q goes to ``q_out`` [M, Hq*hd], k and v straight into the paged cache at ``slot``."""
     _lib.check_rc(_f("artb_decode_finalize_qkv")(
         _lib.ptr(ws), ws.stride(0), M, Hq, Hkv, hd, kpad, _lib.ptr(bias), _lib.ptr(adapter), _lib.ptr(B_all),
-        B_all.stride(0) if B_all is not None else 0, cols, _lib.ptr(pos), theta, _lib.ptr(slot), _lib.ptr(k_cache),
+        B_all.stride(0) if B_all is not None else 0, cols, _lib.ptr(pos), theta, _lib.ptr(q_norm), _lib.ptr(k_norm), eps,
+        _lib.ptr(slot), _lib.ptr(k_cache),
         _lib.ptr(v_cache), _lib.ptr(q_out), q_out.stride(0), _cache_slots(k_cache), _lib.ptr(_lib.status_word(ws.device)),
         _lib.stream_ptr()), "decode_finalize_qkv")
 
