@@ -4,10 +4,13 @@
 // activation matrix and one skinny one:
 //     dB_cat[N, R]   += dY[M, N]^T * T[M, R]          (T = X A^T, saved by the forward)
 //     dA_cat^T[K, R] += X[M, K]^T  * dT[M, R]         (dT = dY (sB))
-// R is the padded LoRA width (64).  The op reads the wide matrix exactly once and does
+// R is the padded LoRA width (64), of which the caller says how many columns are used (rank times modules: 8 to 24
+// mostly): only those are multiplied and added, in steps of 16.  The op reads the wide matrix exactly once and does
 // R/8 times fewer FLOPs than a square GEMM, so it is bandwidth-bound; warp-level
 // mma.sync (m16n8k16) with ldmatrix.trans from padded shared tiles is enough to keep up
-// with HBM.  Token-dimension splits accumulate with fp32 atomics.
+// with HBM.  Token-dimension splits accumulate with fp32 atomics, two columns each: with all 64 columns added one by
+// one they took longer than the loads of short batches (mean of a layer's eight: 18.6 -> 12 us for 2048 rows of the 7B
+// shape, 109 -> 68 for 16 384, of which the bytes take 8 and 50).
 //
 // Counterpart in the reference: autograd through the PEFT/Unsloth LoRA modules
 // (src/art/local/state.py:86-92, backward driven from src/art/local/train.py via HF Trainer).
@@ -23,7 +26,7 @@ constexpr int WG_BC = 128;   // columns of P per CTA
 constexpr int WG_R = 64;     // columns of Q
 constexpr int WG_BM = 32;    // token rows per pipeline chunk
 constexpr int WG_PLD = WG_BC + 8;
-constexpr int WG_QLD = WG_R + 8;
+constexpr int WG_STAGES = 3;
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
   const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
@@ -48,12 +51,15 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// NB: 16-column blocks of Q that are used
+template <int NB>
 __global__ void __launch_bounds__(128)
 lora_wgrad_kernel(const __nv_bfloat16* __restrict__ P, int ldp, const __nv_bfloat16* __restrict__ Q, int ldq,
                   float* __restrict__ out, int ldo, int M, int C, int rows_per_split,
                   const int* __restrict__ seg_off, long out_stride) {
-  __shared__ __align__(16) __nv_bfloat16 sP[2][WG_BM][WG_PLD];
-  __shared__ __align__(16) __nv_bfloat16 sQ[2][WG_BM][WG_QLD];
+  constexpr int QLD = NB * 16 + 8;
+  __shared__ __align__(16) __nv_bfloat16 sP[WG_STAGES][WG_BM][WG_PLD];
+  __shared__ __align__(16) __nv_bfloat16 sQ[WG_STAGES][WG_BM][QLD];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int c0 = blockIdx.x * WG_BC;
   int m_begin = blockIdx.y * rows_per_split;
@@ -80,10 +86,8 @@ lora_wgrad_kernel(const __nv_bfloat16* __restrict__ P, int ldp, const __nv_bfloa
       const bool ok = gm < m_end && gc < C;
       cp_async16(&sP[stage][r][cv * 8], P + (ok ? static_cast<size_t>(gm) * ldp + gc : 0), ok);
     }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {  // Q: 32 rows x 8 vec
-      const int v = tid + i * 128;
-      const int r = v >> 3, cv = v & 7;
+    for (int v = tid; v < WG_BM * NB * 2; v += 128) {  // Q: 32 rows x 2 NB vec
+      const int r = v / (NB * 2), cv = v % (NB * 2);
       const int gm = m0 + r;
       const bool ok = gm < m_end;
       cp_async16(&sQ[stage][r][cv * 8], Q + (ok ? static_cast<size_t>(gm) * ldq + cv * 8 : 0), ok);
@@ -91,24 +95,27 @@ lora_wgrad_kernel(const __nv_bfloat16* __restrict__ P, int ldp, const __nv_bfloa
     cp_async_commit();
   };
 
-  float acc[2][8][4];
+  float acc[2][2 * NB][4];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
+    for (int j = 0; j < 2 * NB; ++j)
 #pragma unroll
       for (int k = 0; k < 4; ++k) acc[i][j][k] = 0.f;
 
   load_chunk(0, 0);
+  if (chunks > 1)
+    load_chunk(1, 1);
+  else
+    cp_async_commit();
+  int st = 0;
   for (int ch = 0; ch < chunks; ++ch) {
-    const int st = ch & 1;
-    if (ch + 1 < chunks) {
-      load_chunk(ch + 1, st ^ 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
+    cp_async_wait<1>();
+    __syncthreads();             // the chunk has arrived, and everyone is done with the stage that is filled next
+    if (ch + 2 < chunks)
+      load_chunk(ch + 2, st == 0 ? 2 : st - 1);
+    else
+      cp_async_commit();
     const int j = lane >> 3, rr = lane & 7;  // ldmatrix: lane supplies row rr of matrix j
 #pragma unroll
     for (int ks = 0; ks < WG_BM / 16; ++ks) {
@@ -123,7 +130,7 @@ lora_wgrad_kernel(const __nv_bfloat16* __restrict__ P, int ldp, const __nv_bfloa
         ldmatrix_x4_trans(a[mi], &sP[st][krow][ccol]);
       }
 #pragma unroll
-      for (int nb = 0; nb < 4; ++nb) {
+      for (int nb = 0; nb < NB; ++nb) {
         // B = Q tile [k][n] -> transposed load gives the col-major fragments of two n8 blocks.
         uint32_t b[4];
         const int krow = k0 + (j & 1) * 8 + rr;
@@ -136,49 +143,63 @@ lora_wgrad_kernel(const __nv_bfloat16* __restrict__ P, int ldp, const __nv_bfloa
         }
       }
     }
-    __syncthreads();
+    st = st == WG_STAGES - 1 ? 0 : st + 1;
   }
+  const bool pairs = !(ldo & 1) && !(reinterpret_cast<uintptr_t>(out) & 7);
+  auto add2 = [&](float* p, float a, float b) {
+    if (pairs) {
+      atomicAdd(reinterpret_cast<float2*>(p), make_float2(a, b));
+    } else {
+      atomicAdd(p, a);
+      atomicAdd(p + 1, b);
+    }
+  };
   const int g = lane >> 2, t = lane & 3;
 #pragma unroll
   for (int mi = 0; mi < 2; ++mi) {
 #pragma unroll
-    for (int nj = 0; nj < 8; ++nj) {
+    for (int nj = 0; nj < 2 * NB; ++nj) {
       const int col = nj * 8 + 2 * t;
       const int r0 = c0 + warp * 32 + mi * 16 + g;
-      if (r0 < C) {
-        atomicAdd(out + static_cast<size_t>(r0) * ldo + col, acc[mi][nj][0]);
-        atomicAdd(out + static_cast<size_t>(r0) * ldo + col + 1, acc[mi][nj][1]);
-      }
-      if (r0 + 8 < C) {
-        atomicAdd(out + static_cast<size_t>(r0 + 8) * ldo + col, acc[mi][nj][2]);
-        atomicAdd(out + static_cast<size_t>(r0 + 8) * ldo + col + 1, acc[mi][nj][3]);
-      }
+      if (r0 < C) add2(out + static_cast<size_t>(r0) * ldo + col, acc[mi][nj][0], acc[mi][nj][1]);
+      if (r0 + 8 < C) add2(out + static_cast<size_t>(r0 + 8) * ldo + col, acc[mi][nj][2], acc[mi][nj][3]);
     }
   }
+}
+
+static int launch_wgrad(dim3 grid, const void* P, int ldp, const void* Q, int ldq, float* out, int ldo, int M, int C, int cols,
+                        int rows_per_split, const int* seg_off, long out_stride, cudaStream_t st) {
+  auto go = [&](auto kern) {
+    kern<<<grid, 128, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(P), ldp, reinterpret_cast<const __nv_bfloat16*>(Q), ldq, out,
+                               ldo, M, C, rows_per_split, seg_off, out_stride);
+    return static_cast<int>(cudaGetLastError());
+  };
+  if (cols <= 16) return go(lora_wgrad_kernel<1>);
+  if (cols <= 32) return go(lora_wgrad_kernel<2>);
+  return go(lora_wgrad_kernel<4>);
 }
 
 }  // namespace artb
 
 using namespace artb;
 
-// out[C, 64] (fp32, ld = ldo) += P[M, C]^T Q[M, 64].  C % 8 == 0; P, Q 16-byte aligned rows.
-ARTB_EXPORT int artb_lora_wgrad(const void* P, int ldp, const void* Q, int ldq, float* out, int ldo, int M, int C,
+// out[C, 64] (fp32, ld = ldo) += P[M, C]^T Q[M, 64].  C % 8 == 0; P, Q 16-byte aligned rows.  Columns of Q from `cols` on are
+// zero or not wanted: what is added to their sums is unspecified.
+ARTB_EXPORT int artb_lora_wgrad(const void* P, int ldp, const void* Q, int ldq, float* out, int ldo, int M, int C, int cols,
                                 cudaStream_t st) {
   if (M <= 0 || C <= 0) return 0;
-  if ((C & 7) || (ldp & 7) || (ldq & 7) || ldo < WG_R) return ERR_BAD_SHAPE;
+  if ((C & 7) || (ldp & 7) || (ldq & 7) || ldo < WG_R || cols <= 0 || cols > WG_R) return ERR_BAD_SHAPE;
+  // five CTAs (40 KB of shared memory at most) per SM keep 80 KB of loads in flight; a split of 64 rows still has two chunks
   const int cblocks = (C + WG_BC - 1) / WG_BC;
-  int splits = (4 * sm_count() + cblocks - 1) / cblocks;
-  const int max_splits = (M + 4 * WG_BM - 1) / (4 * WG_BM);
+  int splits = (5 * sm_count() + cblocks - 1) / cblocks;
+  const int max_splits = (M + 2 * WG_BM - 1) / (2 * WG_BM);
   if (splits > max_splits) splits = max_splits;
   if (splits < 1) splits = 1;
   int rows = (M + splits - 1) / splits;
   rows = (rows + WG_BM - 1) / WG_BM * WG_BM;
   splits = (M + rows - 1) / rows;
   dim3 grid(cblocks, splits);
-  lora_wgrad_kernel<<<grid, 128, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(P), ldp,
-                                          reinterpret_cast<const __nv_bfloat16*>(Q), ldq, out, ldo, M, C, rows,
-                                          nullptr, 0);
-  return static_cast<int>(cudaGetLastError());
+  return launch_wgrad(grid, P, ldp, Q, ldq, out, ldo, M, C, cols, rows, nullptr, 0, st);
 }
 
 
@@ -186,12 +207,9 @@ ARTB_EXPORT int artb_lora_wgrad(const void* P, int ldp, const void* Q, int ldq, 
 // seg_e = rows seg_off[e] .. seg_off[e+1] (device array, padded rows are zero).  One launch covers all experts.
 ARTB_EXPORT int artb_lora_wgrad_grouped(const void* P, int ldp, const void* Q, int ldq, float* out, int ldo,
                                         long out_stride, const int* seg_off, int num_experts, int C, int splits,
-                                        int rows, cudaStream_t st) {
+                                        int rows, int cols, cudaStream_t st) {
   if (num_experts <= 0 || C <= 0 || rows <= 0) return 0;
-  if ((C & 7) || (ldp & 7) || (ldq & 7) || ldo < WG_R || splits < 1) return ERR_BAD_SHAPE;
+  if ((C & 7) || (ldp & 7) || (ldq & 7) || ldo < WG_R || splits < 1 || cols <= 0 || cols > WG_R) return ERR_BAD_SHAPE;
   dim3 grid((C + WG_BC - 1) / WG_BC, splits, num_experts);
-  lora_wgrad_kernel<<<grid, 128, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(P), ldp,
-                                          reinterpret_cast<const __nv_bfloat16*>(Q), ldq, out, ldo, rows, C, 0, seg_off,
-                                          out_stride);
-  return static_cast<int>(cudaGetLastError());
+  return launch_wgrad(grid, P, ldp, Q, ldq, out, ldo, rows, C, cols, 0, seg_off, out_stride, st);
 }

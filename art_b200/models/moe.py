@@ -97,8 +97,9 @@ class GroupedLoraLinear:
     def backward(self, dy, xp, T, plan):
         if self.active and T is not None:
             dT = moe_ops.grouped_gemm(dy, self.B_allT, plan, KPAD)
-            moe_ops.grouped_wgrad(self.dA_acc, xp, dT, plan)
-            moe_ops.grouped_wgrad(self.dB_acc, dy, T, plan)
+            cols = (1 + max(slot for _, _, slot in self.members)) * self.r
+            moe_ops.grouped_wgrad(self.dA_acc, xp, dT, plan, cols=cols)
+            moe_ops.grouped_wgrad(self.dB_acc, dy, T, plan, cols=cols)
             return moe_ops.grouped_gemm(dy, self.WT, plan, self.K, a2=dT, b2=self.A_allT)
         return moe_ops.grouped_gemm(dy, self.WT, plan, self.K)
 

@@ -66,6 +66,7 @@ class LoraLinear:
         dev = self.W.device
         self.active = len(members) > 0
         self.kpad = max(LORA_KPAD, ((len(members) * r + 63) // 64) * 64)
+        self.cols = (1 + max((m.slot for m in members), default=0)) * r       # columns that a member's factors take
         if self.active:
             self.A_cat = torch.zeros(self.kpad, K, dtype=torch.bfloat16, device=dev)
             self.B_cat = torch.zeros(N, self.kpad, dtype=torch.bfloat16, device=dev)
@@ -117,8 +118,8 @@ class LoraLinear:
         if self.active and T is not None:
             dT = skinny_gemm(dy, self.B_catT)                   # [M, kpad]
             # LoRA factor gradients: skinny contractions over the token dimension
-            lora_wgrad(self.dA_acc, x, dT)     # dA_cat^T [K, kpad] += X^T dT
-            lora_wgrad(self.dB_acc, dy, T)     # dB_cat   [N, kpad] += dY^T T
+            lora_wgrad(self.dA_acc, x, dT, cols=self.cols)     # dA_cat^T [K, kpad] += X^T dT
+            lora_wgrad(self.dB_acc, dy, T, cols=self.cols)     # dB_cat   [N, kpad] += dY^T T
             if need_dx:
                 return gemm_tn(dy, self.WT, a2=dT, b2=self.A_catT, residual=dx_residual, swiglu_bwd_gu=swiglu_gu)
             return None
@@ -127,11 +128,11 @@ class LoraLinear:
         return None
 
 
-def lora_wgrad(acc: torch.Tensor, p: torch.Tensor, q: torch.Tensor, transpose_out: bool = False) -> None:
+def lora_wgrad(acc: torch.Tensor, p: torch.Tensor, q: torch.Tensor, transpose_out: bool = False, cols: int | None = None) -> None:
     """``acc += p.T @ q`` (or its transpose) for tall-skinny bf16 operands, fp32 accumulation."""
     from ..ops import wgrad
 
-    wgrad.accumulate(acc, p, q, transpose_out)
+    wgrad.accumulate(acc, p, q, transpose_out, cols)
 
 
 class LoraFlat:

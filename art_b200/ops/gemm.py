@@ -116,7 +116,15 @@ def gemm_tn(a: torch.Tensor, b: torch.Tensor, *, a2: torch.Tensor | None = None,
         raise ValueError("bias must be fp32 [N]")
     st = _lib.status_word(a.device)
     if two_cta is None:
-        two_cta = TWO_CTA_DEFAULT and bn == 0 and M >= 1024 and N >= 512   # bn = 224 with two_cta=True: 256 x 224 pair tiles
+        # 128 x 128 tiles of single CTAs where they fit into one wave: pairs would leave half of the chip idle or more
+        # (2048 x 896, K = 9728: 32 pair tiles, 57 us; 112 single ones, 50)
+        two_cta = TWO_CTA_DEFAULT and bn == 0 and M >= 1024 and N >= 512 and -(-M // 128) * -(-N // 128) > 148
+        if two_cta:
+            # up to three waves: narrower pair tiles where their waves are shorter (2048 x 3584: 112 tiles of 256 columns
+            # or 128 of 224, two waves both ways)
+            pairs = -(-M // 256) * -(-N // 256)
+            if pairs <= 222 and -(-pairs // 74) * 256 > -(-(-(-M // 256) * -(-N // 224)) // 74) * 224:
+                bn = 224        # with two_cta: 256 x 224 pair tiles
     if two_cta:
         rc = _fn2()(
             _lib.ptr(a), a.stride(0), _lib.ptr(b), b.stride(0),
@@ -253,11 +261,13 @@ def skinny_gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = Non
     N = b.shape[0]
     if N > 64 or M < 2048 or K < 1024 or SKINNY_SPLITS <= 1:
         return gemm_tn(a, b, out=out)
+    # at least about one work item per SM: 2048 rows are 16 tiles, of which four slices left most of the chip idle
+    splits = max(SKINNY_SPLITS, min(148 // ((M + 127) // 128), K // 512))
     key = (a.device.index, M, N)
     ws = _skinny_ws.get(key)
     if ws is None:
         ws = _skinny_ws[key] = torch.zeros((M, 64), dtype=torch.float32, device=a.device)
     if out is None:
         out = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
-    gemm_splitk_(ws, a, b, 64, SKINNY_SPLITS)
+    gemm_splitk_(ws, a, b, 64, splits)
     return splitk_finalize(ws, out)

@@ -35,7 +35,7 @@ def _k():
         lib.artb_moe_router_bwd.argtypes = [vp, ci, vp, vp, vp, ci, ci, ci, ci, vp, ci, vp]
         lib.artb_gemm_grouped_bf16_tn.argtypes = [vp, ci, vp, ci, vp, ci, vp, ci, ci, vp, ci, vp, ci, vp, ci, ci, ci,
                                                   ci, ci, vp, vp]
-        lib.artb_lora_wgrad_grouped.argtypes = [vp, ci, vp, ci, vp, ci, cl, vp, ci, ci, ci, ci, vp]
+        lib.artb_lora_wgrad_grouped.argtypes = [vp, ci, vp, ci, vp, ci, cl, vp, ci, ci, ci, ci, ci, vp]
         for f in (lib.artb_moe_router, lib.artb_moe_plan, lib.artb_moe_gather, lib.artb_moe_gather_f32, lib.artb_gemm_f32_grouped_tn, lib.artb_moe_combine,
                   lib.artb_moe_router_bwd, lib.artb_gemm_grouped_bf16_tn, lib.artb_lora_wgrad_grouped):
             f.restype = ci
@@ -185,12 +185,14 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, plan: RoutePlan, n_per_expert
     return out
 
 
-def grouped_wgrad(acc: torch.Tensor, p: torch.Tensor, q: torch.Tensor, plan: RoutePlan, splits: int = 2) -> None:
-    """``acc[e] [C, 64] += p[rows of e].T @ q[rows of e]`` for every expert (fp32 accumulation)."""
+def grouped_wgrad(acc: torch.Tensor, p: torch.Tensor, q: torch.Tensor, plan: RoutePlan, splits: int = 2,
+                  cols: int = 64) -> None:
+    """``acc[e] [C, 64] += p[rows of e].T @ q[rows of e]`` for every expert (fp32 accumulation).  ``cols``: columns of ``q``
+    from this one on are zero or not wanted, and those of ``acc`` unspecified."""
     E, C, R = acc.shape
     assert R == 64 and q.shape[1] == 64 and p.shape[1] == C and acc.is_contiguous()
     _lib.check_rc(_k().artb_lora_wgrad_grouped(_lib.ptr(p), p.stride(0), _lib.ptr(q), q.stride(0), _lib.ptr(acc), R,
-                                               C * R, _lib.ptr(plan.seg_off), E, C, splits, min(p.shape[0], q.shape[0]),
+                                               C * R, _lib.ptr(plan.seg_off), E, C, splits, min(p.shape[0], q.shape[0]), cols,
                                                _lib.stream_ptr()),
                   "lora_wgrad_grouped")
 
