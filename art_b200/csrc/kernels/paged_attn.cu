@@ -93,6 +93,27 @@ __global__ void kv_gather_kernel(const __nv_bfloat16* __restrict__ k_cache, cons
   }
 }
 
+// The cached keys and values at a list of slots -> k | v columns of dst [n, ld], one launch for all sequences of a batch;
+// rows with a negative slot become zeros.
+__global__ void kv_rows_kernel(const __nv_bfloat16* __restrict__ k_cache, const __nv_bfloat16* __restrict__ v_cache,
+                               const int* __restrict__ slot, int n, __nv_bfloat16* __restrict__ dst, int ld, int k_col, int v_col,
+                               int kv_width, long num_slots, int* status) {
+  const int vec = kv_width >> 3;
+  const long total = static_cast<long>(n) * vec;
+  for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < total;
+       i += static_cast<long>(gridDim.x) * blockDim.x) {
+    const int t = i / vec, c = (i % vec) * 8;
+    const int s = slot[t];
+    uint4 k = make_uint4(0, 0, 0, 0), v = k;
+    if (s >= 0 && index_ok(s, num_slots, status)) {
+      k = *reinterpret_cast<const uint4*>(k_cache + static_cast<size_t>(s) * kv_width + c);
+      v = *reinterpret_cast<const uint4*>(v_cache + static_cast<size_t>(s) * kv_width + c);
+    }
+    *reinterpret_cast<uint4*>(dst + static_cast<size_t>(t) * ld + k_col + c) = k;
+    *reinterpret_cast<uint4*>(dst + static_cast<size_t>(t) * ld + v_col + c) = v;
+  }
+}
+
 // ------------------------------------------------------------------ decode attention
 constexpr int PA_KT = 32;  // keys per warp tile
 
@@ -574,6 +595,17 @@ ARTB_EXPORT int artb_kv_gather(const void* k_cache, const void* v_cache, const i
   kv_gather_kernel<<<(unsigned)blocks, 256, 0, st>>>((const bf16*)k_cache, (const bf16*)v_cache, block_table,
                                                     block_size, n_tok, (bf16*)dst, ld, k_col, v_col, kv_width,
                                                     num_blocks, status);
+  return (int)cudaGetLastError();
+}
+
+ARTB_EXPORT int artb_kv_rows(const void* k_cache, const void* v_cache, const int* slot, int n, void* dst, int ld, int k_col,
+                             int v_col, int kv_width, long num_slots, int* status, cudaStream_t st) {
+  if (n <= 0) return 0;
+  if ((kv_width & 7) || (ld & 7) || (k_col & 7) || (v_col & 7)) return ERR_BAD_SHAPE;
+  long blocks = (static_cast<long>(n) * (kv_width / 8) + 255) / 256;
+  if (blocks > 148L * 16) blocks = 148L * 16;
+  kv_rows_kernel<<<(unsigned)blocks, 256, 0, st>>>((const bf16*)k_cache, (const bf16*)v_cache, slot, n, (bf16*)dst, ld, k_col,
+                                                  v_col, kv_width, num_slots, status);
   return (int)cudaGetLastError();
 }
 

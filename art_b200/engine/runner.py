@@ -20,6 +20,7 @@ import math
 import os
 from dataclasses import dataclass
 
+import numpy as np
 import torch
 
 from ..models.config import ModelConfig
@@ -536,7 +537,6 @@ class DeviceRunner:
         while max_blocks < need_blocks:
             max_blocks *= 2
         st = self._decode_state(nb, max_blocks, n_steps)
-        import numpy as np
 
         lens = [len(s.tokens) for s in seqs]
         pad = nb - n
@@ -831,62 +831,78 @@ class NativeRunner(DeviceRunner):
         from ..ops import paged
 
         cfg, dev, bs = self.cfg, self.device, self.kv.shape[1]
-        row_ranges = []
-        tok, pos, gid, adapter, slot, new_rows, last_rows = [], [], [], [], [], [], []
-        cached_spans = []   # (att_row_start, n_cached, blocks)
-        att = 0
-        for i, s in enumerate(seqs):
-            n = len(s.tokens) if s.upto is None else min(s.upto, len(s.tokens))
-            nc = s.num_cached
-            if nc:
-                cached_spans.append((att, nc, s.blocks))
-                gid += [i] * nc
-                att += nc
-            r0 = len(tok)
-            for t in range(nc, n):
-                tok.append(s.tokens[t])
-                pos.append(t)
-                adapter.append(s.adapter)
-                slot.append(s.blocks[t // bs] * bs + t % bs if write_kv else -1)
-                new_rows.append(att)
-                gid.append(i)
-                att += 1
-            row_ranges.append((r0, len(tok)))
-            last_rows.append(len(tok) - 1)
-        M = len(tok)
         Hq, Hkv, hd = cfg.num_heads, cfg.num_kv_heads, cfg.head_dim
+        # the rows of attention: every sequence's cached tokens, then its new ones
+        tok, pos, slot, held, rows, gid, row_ranges, M, att = [], [], [], [], [], [], [], 0, 0
+        for i, s in enumerate(seqs):
+            nc, n = s.num_cached, len(s.tokens) if s.upto is None else min(s.upto, len(s.tokens))
+            new, t = max(0, n - nc), np.arange(max(n, nc))
+            where = np.full(len(t), -1)
+            if write_kv or nc:
+                where = np.asarray(s.blocks)[t // bs] * bs + t % bs
+            tok.append(np.asarray(s.tokens[nc:n], dtype=np.int64))
+            pos.append(t[nc:])
+            slot.append(where[nc:] if write_kv else np.full(new, -1))
+            held.append(where)
+            rows.append(att + t[nc:])
+            gid.append(np.full(len(t), i))
+            row_ranges.append((M, M + new))
+            M, att = M + new, att + len(t)
+        cached = any(s.num_cached for s in seqs)
         step = 128 if hd == 128 else 64         # the tensor-core attention of head dim 128 takes whole 128-query tiles
         S_att = (att + step - 1) // step * step
-        gid += [-(j + 1) for j in range(S_att - att)]
-        any_lora = any(a >= 0 for a in adapter)
-        self._moe_mixed = any_lora and any(a < 0 for a in adapter)
-        t_tok = torch.tensor(tok, dtype=torch.int64, device=dev)
-        t_pos = torch.tensor(pos, dtype=torch.int32, device=dev)
-        t_ad = torch.tensor(adapter, dtype=torch.int32, device=dev)
-        t_slot = torch.tensor(slot, dtype=torch.int32, device=dev)
-        t_gid = torch.tensor(gid, dtype=torch.int32, device=dev)
-        t_rows = torch.tensor(new_rows, dtype=torch.int64, device=dev)
+        gid.append(-1 - np.arange(S_att - att))
+        adapter = np.repeat([s.adapter for s in seqs], [b - a for a, b in row_ranges])
+        any_lora = bool((adapter >= 0).any())
+        self._moe_mixed = any_lora and bool((adapter < 0).any())
+        wide = torch.from_numpy(np.concatenate(tok + rows)).to(dev)
+        t_tok, t_rows = wide[:M], wide[M:]
+        parts = [np.concatenate(p) for p in (pos, slot, held, gid, [adapter])]
+        flat = torch.from_numpy(np.concatenate(parts).astype(np.int32)).to(dev)
+        t_pos, t_slot, t_held, t_gid, t_ad = flat.split([len(p) for p in parts])
         plan = attn_ops.make_plan(t_gid, t_gid, S_att, "native")
-        if cached_spans and step == 128:        # tiles without a new token are not computed
-            plan.wanted = torch.zeros(S_att // step, dtype=torch.uint8, device=dev).index_fill_(0, t_rows // step, 1)
-        # the rows of attention: one buffer for all layers, each of which writes every row that a token has; without cached
-        # tokens the projection's rows are the buffer's first
+        if cached and step == 128:              # tiles without a new token are not computed
+            wanted = np.zeros(S_att // step, dtype=np.uint8)
+            wanted[np.concatenate(rows) // step] = 1
+            plan.wanted = torch.from_numpy(wanted).to(dev)
+        # one buffer for all layers, each of which writes every row that a token has
         buf = torch.empty((S_att, cfg.q_size + 2 * cfg.kv_size), dtype=self.embed.dtype, device=dev)
         buf[att:].zero_()
-        place = not cached_spans and M > 512
+        r0 = int(rows[0][0]) if M and len(rows[0]) else 0
+        run = M > 0 and not cached or len(seqs) == 1        # the new tokens' rows are neighbours
         x = ew.gather_rows(self.embed, t_tok)
-        span_tables = [(a0, nc, torch.tensor(bl, dtype=torch.int32, device=dev)) for a0, nc, bl in cached_spans]
+
+        def attend(li):
+            """Attention of the new tokens, whose queries are in ``buf``; keys and values as the cache holds them."""
+            paged.kv_rows(self.kv.k[li], self.kv.v[li], t_held, buf, cfg.q_size, cfg.q_size + cfg.kv_size)
+            return new_rows(attn_ops.forward(buf, Hq, Hkv, hd, plan, need_grad=False)[0])
+
+        def new_rows(o):
+            return o[r0:r0 + M] if run else o.index_select(0, t_rows)
+
+        if write_kv and 0 < M <= 512 and self._fused_decode_ok(M):
+            # few rows: the projections are split and finished as in a decode step
+            h, _ = ew.rmsnorm_fwd(x, self.layers[0]["ln1"], cfg.rms_norm_eps, want_rstd=False)
+            q = buf[r0:r0 + M, :cfg.q_size] if run else torch.empty((M, cfg.q_size), dtype=buf.dtype, device=dev)
+            for li, L in enumerate(self.layers):
+                def attend_q():
+                    if not run:
+                        buf[:, :cfg.q_size].index_copy_(0, t_rows, q)
+                    return attend(li)
+                nxt = self.layers[li + 1]["ln1"] if li + 1 < len(self.layers) else None
+                x, h = self._layer_fused(li, L, x, h, nxt, t_pos, t_slot, t_ad, any_lora, q, attend_q)
+            return x, row_ranges
+        place = not cached and M > 512          # the projection's rows are the buffer's first
         for li, L in enumerate(self.layers):
             qkv = self._qkv(L, x, t_pos, t_ad, any_lora, out=buf[:M] if place else None)
             paged.kv_write(qkv, cfg.q_size, cfg.q_size + cfg.kv_size, t_slot, self.kv.k[li], self.kv.v[li])
-            if cached_spans:
-                buf.index_copy_(0, t_rows, qkv[:, :buf.shape[1]])
-                for a0, nc, bt in span_tables:
-                    paged.kv_gather(self.kv.k[li], self.kv.v[li], bt, bs, nc, buf[a0:], cfg.q_size, cfg.q_size + cfg.kv_size)
-            elif not place:
-                buf[:M].copy_(qkv[:, :buf.shape[1]])
-            o, _ = attn_ops.forward(buf, Hq, Hkv, hd, plan, need_grad=False)
-            o = o.index_select(0, t_rows) if cached_spans else o[:M]
+            if cached:
+                buf[:, :cfg.q_size].index_copy_(0, t_rows, qkv[:, :cfg.q_size])
+                o = attend(li)
+            else:
+                if not place:
+                    buf[:M].copy_(qkv[:, :buf.shape[1]])
+                o = new_rows(attn_ops.forward(buf, Hq, Hkv, hd, plan, need_grad=False)[0])
             x2 = self._reduce(L["o"](o, t_ad, any_lora, residual=self._res(x)))
             x = self._mlp(L, x2, t_ad, any_lora)
         return x, row_ranges
@@ -927,7 +943,9 @@ class NativeRunner(DeviceRunner):
                 h, _ = ew.rmsnorm_fwd(x, self.layers[0]["ln1"], cfg.rms_norm_eps, want_rstd=False)
                 for li, L in enumerate(self.layers):
                     nxt = self.layers[li + 1]["ln1"] if li + 1 < len(self.layers) else self.final_norm
-                    x, h = self._layer_decode_fused(li, L, x, h, nxt, st, any_lora)
+                    x, h = self._layer_fused(li, L, x, h, nxt, st["pos"], st["slot"], st["ad"], any_lora, st["q"],
+                                             lambda: paged.paged_decode_even(st["q"], self.kv.k[li], self.kv.v[li], st["bt"], st["ctx"],
+                                                                             Hq, Hkv, hd, st["attn_out"], st["attn_ws"]))
                 hidden = h
             else:
                 for li, L in enumerate(self.layers):
@@ -955,31 +973,33 @@ class NativeRunner(DeviceRunner):
         L = self.layers[0]
         return all(isinstance(L.get(k), EngineLinear) and L[k].cols <= 64 for k in ("qkv", "o", "gu", "down"))
 
-    def _layer_decode_fused(self, li: int, L, x, h, next_norm, st, any_lora: bool):
+    def _layer_fused(self, li: int, L, x, h, next_norm, pos, slot, adapters, any_lora: bool, q, attend):
+        """A layer of a few rows ``x`` whose normed form is ``h``; ``q`` receives the queries, the cache the keys and values,
+        before ``attend()`` gives the attention rows.  Returns the rows after the layer and, with ``next_norm``, their norm."""
         from ..ops import paged
 
         cfg = self.cfg
         M, d = x.shape
-        Hq, Hkv, hd = cfg.num_heads, cfg.num_kv_heads, cfg.head_dim
-        ad = st["ad"] if any_lora else None
+        ad = adapters if any_lora else None
         lin = L["qkv"]
         w = lin.partial_sums(h, any_lora)
-        paged.decode_finalize_qkv(w, M, Hq, Hkv, hd, lin.kpad, st["pos"], cfg.rope_theta, st["slot"], self.kv.k[li],
-                                  self.kv.v[li], st["q"], bias=None if lin.bias_ext is None else lin.bias_ext[:lin.N],
+        paged.decode_finalize_qkv(w, M, cfg.num_heads, cfg.num_kv_heads, cfg.head_dim, lin.kpad, pos, cfg.rope_theta, slot,
+                                  self.kv.k[li], self.kv.v[li], q, bias=None if lin.bias_ext is None else lin.bias_ext[:lin.N],
                                   adapter=ad, B_all=lin.B_T, cols=lin.cols, q_norm=L["q_norm"] if cfg.qk_norm else None,
                                   k_norm=L["k_norm"] if cfg.qk_norm else None, eps=cfg.rms_norm_eps)
-        paged.paged_decode_even(st["q"], self.kv.k[li], self.kv.v[li], st["bt"], st["ctx"], Hq, Hkv, hd, st["attn_out"], st["attn_ws"])
+        o = attend()
         lin = L["o"]
-        w = lin.partial_sums(st["attn_out"], any_lora)
+        w = lin.partial_sums(o, any_lora)
         x2, h2 = torch.empty_like(x), torch.empty_like(x)
         paged.decode_finalize_norm(w, M, d, lin.kpad, x2, bias=None if lin.bias_ext is None else lin.bias_ext[:d],
                                    residual=x, adapter=ad, B_all=lin.B_T, cols=lin.cols, norm_w=L["ln2"],
                                    eps=cfg.rms_norm_eps, h_out=h2)
         hact = torch.empty((M, cfg.intermediate_size), dtype=x.dtype, device=x.device)
-        L["gu"](h2, st["ad"], any_lora, swiglu_out=hact)
+        L["gu"](h2, adapters, any_lora, swiglu_out=hact)
         lin = L["down"]
         w = lin.partial_sums(hact, any_lora)
-        x3, h3 = torch.empty_like(x), torch.empty_like(x)
+        x3 = torch.empty_like(x)
+        h3 = torch.empty_like(x) if next_norm is not None else None
         paged.decode_finalize_norm(w, M, d, lin.kpad, x3, bias=None if lin.bias_ext is None else lin.bias_ext[:d],
                                    residual=x2, adapter=ad, B_all=lin.B_T, cols=lin.cols, norm_w=next_norm,
                                    eps=cfg.rms_norm_eps, h_out=h3)

@@ -12,6 +12,7 @@ vp, ci, cl = ctypes.c_void_p, ctypes.c_int, ctypes.c_long
 _sigs = {
     "artb_kv_write": [vp, ci, ci, ci, vp, vp, vp, ci, ci, cl, vp, vp],
     "artb_kv_gather": [vp, vp, vp, ci, ci, vp, ci, ci, ci, ci, cl, vp, vp],
+    "artb_kv_rows": [vp, vp, vp, ci, vp, ci, ci, ci, ci, cl, vp, vp],
     "artb_paged_decode_even": [vp, ci, vp, vp, vp, ci, vp, ci, ci, ci, ci, ci, vp, ci, vp, cl, vp, vp],
     "artb_paged_decode_even_bytes": [ci, ci, ci, ci],
     "artb_paged_decode": [vp, ci, vp, vp, vp, ci, vp, ci, ci, ci, ci, ci, vp, ci, vp, ci, cl, vp, vp],
@@ -98,6 +99,13 @@ def kv_gather(k_cache: torch.Tensor, v_cache: torch.Tensor, block_table_row: tor
     _lib.check_rc(_f("artb_kv_gather")(_lib.ptr(k_cache), _lib.ptr(v_cache), _lib.ptr(block_table_row), block_size,
                                        n_tok, _lib.ptr(dst), dst.stride(0), k_col, v_col, kv_width, k_cache.shape[0],
                                        _lib.ptr(_lib.status_word(dst.device)), _lib.stream_ptr()), "kv_gather")
+
+
+def kv_rows(k_cache: torch.Tensor, v_cache: torch.Tensor, slot: torch.Tensor, dst: torch.Tensor, k_col: int, v_col: int) -> None:
+    """The cached keys and values at ``slot`` (int32 [n]) into the k and v columns of ``dst[:n]``; zeros where negative."""
+    _lib.check_rc(_f("artb_kv_rows")(_lib.ptr(k_cache), _lib.ptr(v_cache), _lib.ptr(slot), slot.numel(), _lib.ptr(dst), dst.stride(0),
+                                     k_col, v_col, k_cache.shape[-2] * k_cache.shape[-1], _cache_slots(k_cache),
+                                     _lib.ptr(_lib.status_word(dst.device)), _lib.stream_ptr()), "kv_rows")
 
 
 def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,
