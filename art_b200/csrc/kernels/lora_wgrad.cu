@@ -27,6 +27,7 @@ constexpr int WG_R = 64;     // columns of Q
 constexpr int WG_BM = 32;    // token rows per pipeline chunk
 constexpr int WG_PLD = WG_BC + 8;
 constexpr int WG_STAGES = 3;
+constexpr int WG_CTAS = 5;   // per SM (40 KB of shared memory at most): 80 KB of loads in flight
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
   const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
@@ -51,17 +52,28 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// NB: 16-column blocks of Q that are used
+struct WgArgs {
+  const __nv_bfloat16 *P, *Q;
+  float* out;
+  int ldp, ldq, ldo, C, cblocks, rows_per_split;
+};
+
+// NB: 16-column blocks of Q that are used.  Two contractions over the same M rows share a launch: CTAs from a.cblocks on
+// belong to b.
 template <int NB>
 __global__ void __launch_bounds__(128)
-lora_wgrad_kernel(const __nv_bfloat16* __restrict__ P, int ldp, const __nv_bfloat16* __restrict__ Q, int ldq,
-                  float* __restrict__ out, int ldo, int M, int C, int rows_per_split,
-                  const int* __restrict__ seg_off, long out_stride) {
+lora_wgrad_kernel(const WgArgs a, const WgArgs b, int M, const int* __restrict__ seg_off, long out_stride) {
   constexpr int QLD = NB * 16 + 8;
   __shared__ __align__(16) __nv_bfloat16 sP[WG_STAGES][WG_BM][WG_PLD];
   __shared__ __align__(16) __nv_bfloat16 sQ[WG_STAGES][WG_BM][QLD];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int c0 = blockIdx.x * WG_BC;
+  const bool second = static_cast<int>(blockIdx.x) >= a.cblocks;
+  const __nv_bfloat16* __restrict__ P = second ? b.P : a.P;
+  const __nv_bfloat16* __restrict__ Q = second ? b.Q : a.Q;
+  float* __restrict__ out = second ? b.out : a.out;
+  const int ldp = second ? b.ldp : a.ldp, ldq = second ? b.ldq : a.ldq, ldo = second ? b.ldo : a.ldo, C = second ? b.C : a.C;
+  const int rows_per_split = second ? b.rows_per_split : a.rows_per_split;
+  const int c0 = (blockIdx.x - (second ? a.cblocks : 0)) * WG_BC;
   int m_begin = blockIdx.y * rows_per_split;
   int m_end = min(M, m_begin + rows_per_split);
   if (seg_off) {
@@ -167,11 +179,26 @@ lora_wgrad_kernel(const __nv_bfloat16* __restrict__ P, int ldp, const __nv_bfloa
   }
 }
 
-static int launch_wgrad(dim3 grid, const void* P, int ldp, const void* Q, int ldq, float* out, int ldo, int M, int C, int cols,
-                        int rows_per_split, const int* seg_off, long out_stride, cudaStream_t st) {
+static WgArgs wg_args(const void* P, int ldp, const void* Q, int ldq, float* out, int ldo, int C) {
+  return WgArgs{reinterpret_cast<const __nv_bfloat16*>(P), reinterpret_cast<const __nv_bfloat16*>(Q), out, ldp, ldq, ldo, C,
+                (C + WG_BC - 1) / WG_BC, 0};
+}
+
+// rows of a split, so that `ctas` CTAs share a contraction over M rows; a split of 64 rows still has two chunks
+static int wg_split(WgArgs& a, int M, int ctas) {
+  int splits = (ctas + a.cblocks - 1) / a.cblocks;
+  const int max_splits = (M + 2 * WG_BM - 1) / (2 * WG_BM);
+  if (splits > max_splits) splits = max_splits;
+  if (splits < 1) splits = 1;
+  const int rows = (M + splits - 1) / splits;
+  a.rows_per_split = (rows + WG_BM - 1) / WG_BM * WG_BM;
+  return (M + a.rows_per_split - 1) / a.rows_per_split;
+}
+
+static int launch_wgrad(dim3 grid, const WgArgs& a, const WgArgs& b, int M, int cols, const int* seg_off, long out_stride,
+                        cudaStream_t st) {
   auto go = [&](auto kern) {
-    kern<<<grid, 128, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(P), ldp, reinterpret_cast<const __nv_bfloat16*>(Q), ldq, out,
-                               ldo, M, C, rows_per_split, seg_off, out_stride);
+    kern<<<grid, 128, 0, st>>>(a, b, M, seg_off, out_stride);
     return static_cast<int>(cudaGetLastError());
   };
   if (cols <= 16) return go(lora_wgrad_kernel<1>);
@@ -189,19 +216,26 @@ ARTB_EXPORT int artb_lora_wgrad(const void* P, int ldp, const void* Q, int ldq, 
                                 cudaStream_t st) {
   if (M <= 0 || C <= 0) return 0;
   if ((C & 7) || (ldp & 7) || (ldq & 7) || ldo < WG_R || cols <= 0 || cols > WG_R) return ERR_BAD_SHAPE;
-  // five CTAs (40 KB of shared memory at most) per SM keep 80 KB of loads in flight; a split of 64 rows still has two chunks
-  const int cblocks = (C + WG_BC - 1) / WG_BC;
-  int splits = (5 * sm_count() + cblocks - 1) / cblocks;
-  const int max_splits = (M + 2 * WG_BM - 1) / (2 * WG_BM);
-  if (splits > max_splits) splits = max_splits;
-  if (splits < 1) splits = 1;
-  int rows = (M + splits - 1) / splits;
-  rows = (rows + WG_BM - 1) / WG_BM * WG_BM;
-  splits = (M + rows - 1) / rows;
-  dim3 grid(cblocks, splits);
-  return launch_wgrad(grid, P, ldp, Q, ldq, out, ldo, M, C, cols, rows, nullptr, 0, st);
+  WgArgs a = wg_args(P, ldp, Q, ldq, out, ldo, C);
+  const int splits = wg_split(a, M, WG_CTAS * sm_count());
+  return launch_wgrad(dim3(a.cblocks, splits), a, a, M, cols, nullptr, 0, st);
 }
 
+// Both factor gradients of a projection in one launch: out1[C1, 64] += P1^T Q1 and out2[C2, 64] += P2^T Q2 over M rows.
+ARTB_EXPORT int artb_lora_wgrad_pair(const void* P1, int ldp1, const void* Q1, int ldq1, float* out1, int ldo1, int C1,
+                                     const void* P2, int ldp2, const void* Q2, int ldq2, float* out2, int ldo2, int C2, int M,
+                                     int cols, cudaStream_t st) {
+  if (M <= 0) return 0;
+  if (C1 <= 0 || C2 <= 0 || (C1 & 7) || (C2 & 7) || (ldp1 & 7) || (ldq1 & 7) || (ldp2 & 7) || (ldq2 & 7) || ldo1 < WG_R ||
+      ldo2 < WG_R || cols <= 0 || cols > WG_R)
+    return ERR_BAD_SHAPE;
+  WgArgs a = wg_args(P1, ldp1, Q1, ldq1, out1, ldo1, C1), b = wg_args(P2, ldp2, Q2, ldq2, out2, ldo2, C2);
+  // splits of about the same number of rows on both sides
+  const int all = a.cblocks + b.cblocks, ctas = WG_CTAS * sm_count();
+  const int sa = wg_split(a, M, static_cast<int>(static_cast<long>(ctas) * a.cblocks / all));
+  const int sb = wg_split(b, M, static_cast<int>(static_cast<long>(ctas) * b.cblocks / all));
+  return launch_wgrad(dim3(all, sa > sb ? sa : sb), a, b, M, cols, nullptr, 0, st);
+}
 
 // Grouped form for expert-sorted rows: out[e][C, 64] += P[seg_e, C]^T Q[seg_e, 64] for every expert e,
 // seg_e = rows seg_off[e] .. seg_off[e+1] (device array, padded rows are zero).  One launch covers all experts.
@@ -210,6 +244,6 @@ ARTB_EXPORT int artb_lora_wgrad_grouped(const void* P, int ldp, const void* Q, i
                                         int rows, int cols, cudaStream_t st) {
   if (num_experts <= 0 || C <= 0 || rows <= 0) return 0;
   if ((C & 7) || (ldp & 7) || (ldq & 7) || ldo < WG_R || splits < 1 || cols <= 0 || cols > WG_R) return ERR_BAD_SHAPE;
-  dim3 grid((C + WG_BC - 1) / WG_BC, splits, num_experts);
-  return launch_wgrad(grid, P, ldp, Q, ldq, out, ldo, rows, C, cols, 0, seg_off, out_stride, st);
+  const WgArgs a = wg_args(P, ldp, Q, ldq, out, ldo, C);
+  return launch_wgrad(dim3(a.cblocks, splits, num_experts), a, a, rows, cols, seg_off, out_stride, st);
 }

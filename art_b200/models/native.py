@@ -33,6 +33,7 @@ import torch
 
 from ..ops import attention as attn_ops
 from ..ops import elementwise as ew
+from ..ops import wgrad
 from ..ops.gemm import gemm_tn, skinny_gemm
 from ..ops.lora_pack import LoraTable
 from .config import ModelConfig
@@ -118,8 +119,8 @@ class LoraLinear:
         if self.active and T is not None:
             dT = skinny_gemm(dy, self.B_catT)                   # [M, kpad]
             # LoRA factor gradients: skinny contractions over the token dimension
-            lora_wgrad(self.dA_acc, x, dT, cols=self.cols)     # dA_cat^T [K, kpad] += X^T dT
-            lora_wgrad(self.dB_acc, dy, T, cols=self.cols)     # dB_cat   [N, kpad] += dY^T T
+            # dA_cat^T [K, kpad] += X^T dT ;  dB_cat [N, kpad] += dY^T T
+            wgrad.accumulate_pair(self.dA_acc, x, dT, self.dB_acc, dy, T, cols=self.cols)
             if need_dx:
                 return gemm_tn(dy, self.WT, a2=dT, b2=self.A_catT, residual=dx_residual, swiglu_bwd_gu=swiglu_gu)
             return None

@@ -9,6 +9,27 @@ import torch
 from . import _lib
 
 _fn = None
+_fn_pair = None
+
+
+def accumulate_pair(acc1: torch.Tensor, p1: torch.Tensor, q1: torch.Tensor, acc2: torch.Tensor, p2: torch.Tensor, q2: torch.Tensor,
+                    cols: int | None = None) -> None:
+    """:func:`accumulate` for both factors of a projection, over the same rows, in one launch."""
+    global _fn_pair
+    if not p1.is_cuda or q1.shape[1] != 64:
+        accumulate(acc1, p1, q1, cols=cols)
+        accumulate(acc2, p2, q2, cols=cols)
+        return
+    if _fn_pair is None:
+        _fn_pair = _lib.kernels().artb_lora_wgrad_pair
+        vp, ci = ctypes.c_void_p, ctypes.c_int
+        _fn_pair.argtypes = [vp, ci, vp, ci, vp, ci, ci] * 2 + [ci, ci, vp]
+        _fn_pair.restype = ci
+    for acc, p in ((acc1, p1), (acc2, p2)):
+        assert acc.dtype == torch.float32 and acc.stride(1) == 1 and acc.shape[0] == p.shape[1] and p.shape[0] == p1.shape[0]
+    _lib.check_rc(_fn_pair(_lib.ptr(p1), p1.stride(0), _lib.ptr(q1), q1.stride(0), _lib.ptr(acc1), acc1.stride(0), p1.shape[1],
+                           _lib.ptr(p2), p2.stride(0), _lib.ptr(q2), q2.stride(0), _lib.ptr(acc2), acc2.stride(0), p2.shape[1],
+                           p1.shape[0], cols or 64, _lib.stream_ptr()), "lora_wgrad_pair")
 
 
 def accumulate(acc: torch.Tensor, p: torch.Tensor, q: torch.Tensor, transpose_out: bool = False,
