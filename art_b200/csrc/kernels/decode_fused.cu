@@ -135,6 +135,22 @@ __device__ __forceinline__ int stage_shrink(float* wrow, int N, int kpad, int co
   return a;
 }
 
+// Before the wait for the product: the row's slice of sB, which no kernel of the step writes, on its way into L2.  The
+// weights that stream through it have pushed it out since the last step, and a row then needs `cols` / 8 dependent trips to
+// memory.  Of a large batch, whose rows share few slots, a row warms a quarter.
+__device__ __forceinline__ void warm_expand(const int* adapter, const __nv_bfloat16* B_all, int ldb, int cols, int N) {
+  if (!adapter) return;
+  const int row = blockIdx.x, a = adapter[row];
+  if (a < 0) return;
+  const __nv_bfloat16* B = B_all + static_cast<size_t>(a) * cols * ldb;
+  const int step = gridDim.x > 64 ? 4 : 1, lines = (N + 63) / 64;
+  for (int i = threadIdx.x; i < cols * lines; i += blockDim.x) {
+    const int j = i / lines, l = i - j * lines;
+    if (step == 1 || ((j + (row >> 2)) & 3) == 0)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(B + static_cast<size_t>(j) * ldb + l * 64));
+  }
+}
+
 }  // namespace
 
 template <int MAX_VEC>
@@ -147,6 +163,7 @@ decode_finalize_norm_kernel(float* __restrict__ ws, int ldw, int N, int kpad, co
   __shared__ float t_s[DF_MAX_COLS];
   __shared__ float red[DF_THREADS / 32];
   pdl_launch_dependents();
+  warm_expand(adapter, B_all, ldb, cols, N);
   pdl_wait();
   const int row = blockIdx.x;
   float* wrow = ws + static_cast<size_t>(row) * ldw;
@@ -202,10 +219,11 @@ decode_finalize_norm_kernel(float* __restrict__ ws, int ldw, int N, int kpad, co
 
 // Columns of the workspace row: [ q: Hq heads | k: Hkv heads | v: Hkv heads | shrink: kpad ], heads of hd values.
 // Rotate-half RoPE: the pair is (i, i + hd/2) inside a head, angle pos * theta^(-2i/hd).
-// 256 threads, two CTAs per SM (128 registers each): the 320 (rope pair | v) units of a 7B row take two short passes
-constexpr int DQ_THREADS = 256;
-
-__global__ void __launch_bounds__(DQ_THREADS, 2)
+// 512 threads while every row has an SM to itself: the (rope pair | v) units of a row (448 of 32 / 8 heads of 128) are then one
+// pass; 64 such rows with 24 low-rank columns took 19 us in two passes and take 11.  Beyond, two CTAs of 256 threads (128
+// registers) per SM: with 320, which make 28 / 4 heads one pass, registers spill (256 rows: 16 -> 19 us).
+template <int DQ_THREADS>
+__global__ void __launch_bounds__(DQ_THREADS, DQ_THREADS == 512 ? 1 : 2)
 decode_finalize_qkv_kernel(float* __restrict__ ws, int ldw, int Hq, int Hkv, int hd, int kpad,
                            const float* __restrict__ bias, const int* __restrict__ adapter,
                            const __nv_bfloat16* __restrict__ B_all, int ldb, int cols, const int* __restrict__ pos,
@@ -215,6 +233,7 @@ decode_finalize_qkv_kernel(float* __restrict__ ws, int ldw, int Hq, int Hkv, int
                            long num_slots, int* status) {
   __shared__ float t_s[DF_MAX_COLS];
   __shared__ float cs_s[128], sn_s[128];     // cos / sin of the row's position for every frequency: shared by all heads
+  warm_expand(adapter, B_all, ldb, cols, (Hq + 2 * Hkv) * hd);
   pdl_wait();                  // attention comes next: its first CTAs would share the few SMs that a product leaves free
   pdl_launch_dependents();
   const int row = blockIdx.x;
@@ -330,12 +349,15 @@ ARTB_EXPORT int artb_decode_finalize_qkv(float* ws, int ldw, int M, int Hq, int 
   if (!q_norm != !k_norm || (q_norm && (hd & (hd - 1)))) return ERR_BAD_SHAPE;
   if (adapter && (cols <= 0 || cols > DF_MAX_COLS || (kpad & 3) || (ldb & 7) || !B_all)) return ERR_BAD_SHAPE;
   if (reinterpret_cast<uintptr_t>(ws) & 15) return ERR_BAD_ALIGN;
-  return static_cast<int>(launch_kernel(
-      decode_finalize_qkv_kernel, dim3(M), dim3(DQ_THREADS), 0, st, ws, ldw, Hq, Hkv, hd, kpad, bias, adapter,
-      reinterpret_cast<const __nv_bfloat16*>(B_all), ldb, cols, pos, log2f(theta),
-      reinterpret_cast<const __nv_bfloat16*>(q_norm), reinterpret_cast<const __nv_bfloat16*>(k_norm), eps, slot,
-      reinterpret_cast<__nv_bfloat16*>(k_cache), reinterpret_cast<__nv_bfloat16*>(v_cache),
-      reinterpret_cast<__nv_bfloat16*>(q_out), ldq, num_slots, status));
+  auto go = [&](auto kern, int threads) {
+    return static_cast<int>(launch_kernel(
+        kern, dim3(M), dim3(threads), 0, st, ws, ldw, Hq, Hkv, hd, kpad, bias, adapter,
+        reinterpret_cast<const __nv_bfloat16*>(B_all), ldb, cols, pos, log2f(theta),
+        reinterpret_cast<const __nv_bfloat16*>(q_norm), reinterpret_cast<const __nv_bfloat16*>(k_norm), eps, slot,
+        reinterpret_cast<__nv_bfloat16*>(k_cache), reinterpret_cast<__nv_bfloat16*>(v_cache),
+        reinterpret_cast<__nv_bfloat16*>(q_out), ldq, num_slots, status));
+  };
+  return M <= sm_count() ? go(decode_finalize_qkv_kernel<512>, 512) : go(decode_finalize_qkv_kernel<256>, 256);
 }
 
 // Programmatic dependent launch for the kernels of the decode step (see pdl_switch in host_utils.h); returns the
