@@ -96,9 +96,15 @@ __device__ __forceinline__ void raster_tile(int tile, int m_tiles, int n_tiles, 
   n = r / rows;
 }
 
-template <int BN, int STAGES>
+// AR: rows of A that a stage holds.  A product of few rows is bound by how much of its weights is in flight, and a full
+// tile of A, all but the first rows of it zeros, takes up to half of a stage; with AR = 16 or 64 (M at most that) the same
+// shared memory holds up to twice the stages.  The MMA still reads 128 rows: those from AR on are whatever lies behind (the
+// stage's B tile, always mapped), and only reach accumulator rows that no epilogue keeps.  22016 x 2048 weights, 8 rows, cold:
+// 37.9 -> 30.7 us; 24576 x 4096, 64 rows, in a decode step: 43 -> 38.
+template <int BN, int STAGES, int AR = GEMM_BM>
 struct GemmSmemLayout {
-  static constexpr int A_BYTES = GEMM_BM * GEMM_BK * 2;
+  static_assert(AR % 8 == 0 && AR <= GEMM_BM && AR + BN >= GEMM_BM, "whole swizzle atoms; 128 rows are readable in a stage");
+  static constexpr int A_BYTES = AR * GEMM_BK * 2;
   static constexpr int B_BYTES = BN * GEMM_BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
@@ -138,13 +144,13 @@ __device__ __forceinline__ auto epi_flush(E& e, int row, int) -> decltype(e.flus
 template <class E>
 __device__ __forceinline__ void epi_flush(E&, int, long) {}
 
-template <int BN, int STAGES, class Sched, class Epi, class Comm = NoComm>
+template <int BN, int STAGES, class Sched, class Epi, class Comm = NoComm, int AR = GEMM_BM>
 __global__ void __launch_bounds__(gemm_pipe_threads<Epi>() + Comm::THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmA2,
                     const __grid_constant__ CUtensorMap tmB2, int kb_main, int kb_extra,
                     Sched sched, Epi epi_in, int* status, Comm comm) {
-  using L = GemmSmemLayout<BN, STAGES>;
+  using L = GemmSmemLayout<BN, STAGES, AR>;
   // two accumulators of BN columns each; the allocation is rounded up to a power of two
   constexpr uint32_t TMEM_COLS = 2 * BN <= 32 ? 32 : 2 * BN <= 64 ? 64 : 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
   static_assert(BN % 32 == 0 && BN <= 256, "BN");

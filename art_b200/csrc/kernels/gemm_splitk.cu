@@ -14,11 +14,12 @@
 
 namespace artb {
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, int AR = GEMM_BM>
 static int launch_splitk(const CUtensorMap& tA, const CUtensorMap& tB, int kb_main, int M, int N, int splits,
                          float* ws, int ldw, int* status, cudaStream_t stream) {
-  using L = GemmSmemLayout<BN, STAGES>;
-  auto kern = gemm_tcgen05_kernel<BN, STAGES, SchedSplitK, EpiAtomic<BN>>;
+  using L = GemmSmemLayout<BN, STAGES, AR>;
+  static_assert(L::TOTAL <= 227 * 1024, "shared memory");
+  auto kern = gemm_tcgen05_kernel<BN, STAGES, SchedSplitK, EpiAtomic<BN>, NoComm, AR>;
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -96,12 +97,19 @@ ARTB_EXPORT int artb_gemm_splitk_bf16_tn(const void* A, int lda, const void* B, 
                                          int N, int K, int bn, int splits, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0 || (K & 7) || (N & 3) || (ldw & 3) || splits < 1) return ERR_BAD_SHAPE;
   if (reinterpret_cast<uintptr_t>(ws) & 15) return ERR_BAD_ALIGN;
+  if (bn != 64 && bn != 128 && bn != 256) return ERR_BAD_SHAPE;
   const int kb_main = (K + GEMM_BK - 1) / GEMM_BK;
   if (splits > kb_main) splits = kb_main;
   CUtensorMap tA, tB;
   int e;
-  if ((e = make_tmap_bf16_2d(&tA, A, M, K, lda, GEMM_BM, GEMM_BK))) return e;
+  // few rows: stages with as many rows of A as there are, and more of them
+  const int ar = bn == 64 || M > 64 ? GEMM_BM : M > 16 ? 64 : 16;
+  if ((e = make_tmap_bf16_2d(&tA, A, M, K, lda, ar, GEMM_BK))) return e;
   if ((e = make_tmap_bf16_2d(&tB, B, N, K, ldb, bn, GEMM_BK))) return e;
+  if (ar == 16 && bn == 256) return launch_splitk<256, 6, 16>(tA, tB, kb_main, M, N, splits, ws, ldw, status, stream);
+  if (ar == 16) return launch_splitk<128, 12, 16>(tA, tB, kb_main, M, N, splits, ws, ldw, status, stream);
+  if (ar == 64 && bn == 256) return launch_splitk<256, 5, 64>(tA, tB, kb_main, M, N, splits, ws, ldw, status, stream);
+  if (ar == 64) return launch_splitk<128, 9, 64>(tA, tB, kb_main, M, N, splits, ws, ldw, status, stream);
   if (bn == 256) return launch_splitk<256, 4>(tA, tB, kb_main, M, N, splits, ws, ldw, status, stream);
   if (bn == 128) return launch_splitk<128, 6>(tA, tB, kb_main, M, N, splits, ws, ldw, status, stream);
   if (bn == 64) return launch_splitk<64, 8>(tA, tB, kb_main, M, N, splits, ws, ldw, status, stream);

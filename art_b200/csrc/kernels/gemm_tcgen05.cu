@@ -19,14 +19,14 @@
 
 namespace artb {
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, int AR = GEMM_BM>
 static int launch_gemm(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tA2,
                        const CUtensorMap& tB2, int kb_main, int kb_extra, int M, int N,
                        const EpiStore<BN>& epi, int* status, int max_ctas, cudaStream_t stream) {
-  using L = GemmSmemLayout<BN, STAGES>;
+  using L = GemmSmemLayout<BN, STAGES, AR>;
   // operand stages + the epilogue warps' 4 KB re-layout slabs (static shared memory) must fit the 227 KB of a CTA
   static_assert(L::TOTAL + 4 * EpiStore<BN>::COL_SPLIT * 4096 + 64 <= 227 * 1024, "shared memory");
-  auto kern = gemm_tcgen05_kernel<BN, STAGES, SchedMFast, EpiStore<BN>>;
+  auto kern = gemm_tcgen05_kernel<BN, STAGES, SchedMFast, EpiStore<BN>, NoComm, AR>;
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -89,12 +89,14 @@ ARTB_EXPORT int artb_gemm_bf16_tn(const void* A, int lda, const void* B, int ldb
   if (bn == 0) bn = artb_pick_bn(M, N, max_ctas > 0 && max_ctas < sm_count() ? max_ctas : sm_count());
   if (bn != 64 && bn != 128 && bn != 160 && bn != 192 && bn != 224 && bn != 256) return ERR_BAD_SHAPE;
 
+  // few rows: stages with as many rows of A as there are, and more of them
+  const int ar = bn < 128 || bn == 224 || M > 64 ? GEMM_BM : M > 16 ? 64 : 16;
   CUtensorMap tA, tB, tA2, tB2;
   int e;
-  if ((e = make_tmap_bf16_2d(&tA, A, M, K, lda, GEMM_BM, GEMM_BK))) return e;
+  if ((e = make_tmap_bf16_2d(&tA, A, M, K, lda, ar, GEMM_BK))) return e;
   if ((e = make_tmap_bf16_2d(&tB, B, N, K, ldb, bn, GEMM_BK))) return e;
   if (K2 > 0) {
-    if ((e = make_tmap_bf16_2d(&tA2, A2, M, K2, lda2, GEMM_BM, GEMM_BK))) return e;
+    if ((e = make_tmap_bf16_2d(&tA2, A2, M, K2, lda2, ar, GEMM_BK))) return e;
     if ((e = make_tmap_bf16_2d(&tB2, B2, N, K2, ldb2, bn, GEMM_BK))) return e;
   } else {
     tA2 = tA;
@@ -103,7 +105,7 @@ ARTB_EXPORT int artb_gemm_bf16_tn(const void* A, int lda, const void* B, int ldb
   const int kb_main = (K + GEMM_BK - 1) / GEMM_BK;
   const int kb_extra = (K2 + GEMM_BK - 1) / GEMM_BK;
 
-#define ARTB_LAUNCH(BN_, ST_)                                                                     \
+#define ARTB_LAUNCH(BN_, ...)                                                                     \
   {                                                                                               \
     EpiStore<BN_> epi{C, reinterpret_cast<const __nv_bfloat16*>(R),                               \
                       reinterpret_cast<__nv_bfloat16*>(H), bias, ldc, ldr, ldh, M, N,              \
@@ -111,8 +113,20 @@ ARTB_EXPORT int artb_gemm_bf16_tn(const void* A, int lda, const void* B, int ldb
                       epilogue == EPI_SWIGLU_BWD ? 1 : 0, epilogue == EPI_RELUGLU ? 1 : 0,        \
                       epilogue == EPI_SILU ? res_cols : 0,                                        \
                       epilogue == EPI_RELU2 ? (res_cols > 0 ? res_cols : N) : 0};                 \
-    return launch_gemm<BN_, ST_>(tA, tB, tA2, tB2, kb_main, kb_extra, M, N, epi, status, max_ctas, \
+    return launch_gemm<BN_, __VA_ARGS__>(tA, tB, tA2, tB2, kb_main, kb_extra, M, N, epi, status, max_ctas, \
                                  stream);                                                         \
+  }
+  if (ar == 16) {
+    if (bn == 256) ARTB_LAUNCH(256, 5, 16)
+    if (bn == 192) ARTB_LAUNCH(192, 7, 16)
+    if (bn == 160) ARTB_LAUNCH(160, 8, 16)
+    ARTB_LAUNCH(128, 10, 16)
+  }
+  if (ar == 64) {
+    if (bn == 256) ARTB_LAUNCH(256, 4, 64)
+    if (bn == 192) ARTB_LAUNCH(192, 6, 64)
+    if (bn == 160) ARTB_LAUNCH(160, 6, 64)
+    ARTB_LAUNCH(128, 8, 64)
   }
   if (bn == 256) ARTB_LAUNCH(256, 4)
   if (bn == 224) ARTB_LAUNCH(224, 4)

@@ -620,16 +620,16 @@ static SamplePlan sample_plan(int M, int V) {
   return best;
 }
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, int AR = GEMM_BM>
 static int launch_sample(const void* H, int ldh, const void* W, int ldw, const SamplePlan& p, const EpiSample<BN>& epi, int K,
                          int* status, cudaStream_t stream) {
-  using L = GemmSmemLayout<BN, STAGES>;
+  using L = GemmSmemLayout<BN, STAGES, AR>;
   static_assert(L::TOTAL <= 227 * 1024, "shared memory");
   CUtensorMap tA, tB;
   int rc;
-  if ((rc = make_tmap_bf16_2d(&tA, H, epi.M, K, ldh, GEMM_BM, GEMM_BK))) return rc;
+  if ((rc = make_tmap_bf16_2d(&tA, H, epi.M, K, ldh, AR, GEMM_BK))) return rc;
   if ((rc = make_tmap_bf16_2d(&tB, W, epi.V, K, ldw, BN, GEMM_BK))) return rc;
-  auto kern = gemm_tcgen05_kernel<BN, STAGES, SchedVocabSpan, EpiSample<BN>>;
+  auto kern = gemm_tcgen05_kernel<BN, STAGES, SchedVocabSpan, EpiSample<BN>, NoComm, AR>;
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -660,6 +660,8 @@ ARTB_EXPORT int artb_sample_partials(const void* H, int ldh, const void* W, int 
   if (lp_pairs(M)) return launch_lp(H, ldh, W, ldw, M, V, K, parts / 2, epi(W256{}), status, stream);
   const SamplePlan p = sample_plan(M, V);
   if (p.bn == 256) return launch_sample<256, 4>(H, ldh, W, ldw, p, epi(W256{}), K, status, stream);
+  if (p.bn == 224 && M <= 16) return launch_sample<224, 7, 16>(H, ldh, W, ldw, p, epi(std::integral_constant<int, 224>{}), K, status, stream);
+  if (p.bn == 224 && M <= 64) return launch_sample<224, 6, 64>(H, ldh, W, ldw, p, epi(std::integral_constant<int, 224>{}), K, status, stream);
   if (p.bn == 224) return launch_sample<224, 5>(H, ldh, W, ldw, p, epi(std::integral_constant<int, 224>{}), K, status, stream);
   return launch_sample<160, 6>(H, ldh, W, ldw, p, epi(std::integral_constant<int, 160>{}), K, status, stream);
 }
