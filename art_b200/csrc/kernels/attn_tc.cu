@@ -24,6 +24,7 @@
 
 #include "host_utils.h"
 #include "ptx_sm100.cuh"
+#include "transpose.cuh"
 
 namespace artb {
 
@@ -407,26 +408,6 @@ attn_tc_fwd_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
   }
 }
 
-// Vt[(kvh * 128 + d), token] = qkv[token, (Hq + Hkv + kvh) * 128 + d]
-__global__ void attn_tc_transpose_v_kernel(const __nv_bfloat16* __restrict__ qkv, int ld, int vcol0,
-                                           __nv_bfloat16* __restrict__ vt, long M, int width) {
-  __shared__ __nv_bfloat16 tile[32][33];
-  const long t0 = static_cast<long>(blockIdx.x) * 32;
-  const int c0 = blockIdx.y * 32;
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const long t = t0 + i;
-    tile[i][threadIdx.x] = (t < M && c0 + static_cast<int>(threadIdx.x) < width)
-                               ? qkv[t * ld + vcol0 + c0 + threadIdx.x]
-                               : __float2bfloat16(0.f);
-  }
-  __syncthreads();
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int c = c0 + i;
-    const long t = t0 + threadIdx.x;
-    if (c < width && t < M) vt[static_cast<size_t>(c) * M + t] = tile[threadIdx.x][i];
-  }
-}
-
 }  // namespace artb
 
 using namespace artb;
@@ -442,10 +423,9 @@ ARTB_EXPORT int artb_attn_tc_fwd(const void* qkv, int ld, const int* gid, const 
   const long M = static_cast<long>(rows) * S;
   if (M > 0x7fffffffL || (M & 7)) return ERR_BAD_SHAPE;
   {
-    dim3 grid(static_cast<unsigned>((M + 31) / 32), (Hkv * TC_HD + 31) / 32), block(32, 8);
-    attn_tc_transpose_v_kernel<<<grid, block, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(qkv), ld,
-                                                       (Hq + Hkv) * TC_HD, reinterpret_cast<__nv_bfloat16*>(vt), M,
-                                                       Hkv * TC_HD);
+    const dim3 grid(static_cast<unsigned>((M + 63) / 64), Hkv * TC_HD / 64);
+    attn_tc_transpose_kernel<<<grid, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(qkv), ld, (Hq + Hkv) * TC_HD,
+                                                   reinterpret_cast<__nv_bfloat16*>(vt), M);
   }
   CUtensorMap tmQK, tmVt;
   int e;

@@ -26,6 +26,7 @@
 
 #include "host_utils.h"
 #include "ptx_sm100.cuh"
+#include "transpose.cuh"
 
 namespace artb {
 
@@ -717,36 +718,6 @@ __global__ void attn_tc_combine_dkv_kernel(const float* __restrict__ partial, in
   }
 }
 
-// dst[c, token] = src[token, c0 + c] for c < width: 64 x 64 tiles, 16-byte loads and stores (M % 8 == 0, width % 64 == 0)
-__global__ void __launch_bounds__(256)
-attn_tc_transpose_kernel(const __nv_bfloat16* __restrict__ src, int ld, int c0, __nv_bfloat16* __restrict__ dst, long M,
-                         int width) {
-  __shared__ __nv_bfloat16 tile[64][64 + 8];
-  const long t0 = static_cast<long>(blockIdx.x) * 64;
-  const int cb = blockIdx.y * 64;
-  const int tid = threadIdx.x;
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int v = tid + i * 256;          // 512 vectors: 64 tokens x 8
-    const int r = v >> 3, cv = v & 7;
-    const long t = t0 + r;
-    uint4 x = make_uint4(0, 0, 0, 0);
-    if (t < M) x = *reinterpret_cast<const uint4*>(src + t * ld + c0 + cb + cv * 8);
-    *reinterpret_cast<uint4*>(&tile[r][cv * 8]) = x;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int v = tid + i * 256;          // 512 vectors: 64 columns x 8 token groups
-    const int c = v >> 3, tv = v & 7;
-    __nv_bfloat16 e[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) e[j] = tile[tv * 8 + j][c];
-    const long t = t0 + tv * 8;
-    if (t < M) *reinterpret_cast<uint4*>(dst + static_cast<size_t>(cb + c) * M + t) = *reinterpret_cast<const uint4*>(e);
-  }
-}
-
 // D[h, m] = sum_d dO[m, h*HD + d] * O[m, h*HD + d]   (one warp per 128 columns of a token: one or two heads)
 template <int HD>
 __global__ void attn_tc_rowdot_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O, int ld,
@@ -792,12 +763,10 @@ static int launch_tc_bwd(const void* qkv, int ld, const void* out, const void* d
         reinterpret_cast<const bf*>(dout), reinterpret_cast<const bf*>(out), ldo, Dbuf, M, Hq);
     const unsigned block = 256;
     dim3 gq(static_cast<unsigned>((M + 63) / 64), Hq * HD / 64), gk(static_cast<unsigned>((M + 63) / 64), Hkv * HD / 64);
-    attn_tc_transpose_kernel<<<gq, block, 0, st>>>(reinterpret_cast<const bf*>(qkv), ld, 0, reinterpret_cast<bf*>(qt), M,
-                                                   Hq * HD);
-    attn_tc_transpose_kernel<<<gq, block, 0, st>>>(reinterpret_cast<const bf*>(dout), ldo, 0, reinterpret_cast<bf*>(dot), M,
-                                                   Hq * HD);
+    attn_tc_transpose_kernel<<<gq, block, 0, st>>>(reinterpret_cast<const bf*>(qkv), ld, 0, reinterpret_cast<bf*>(qt), M);
+    attn_tc_transpose_kernel<<<gq, block, 0, st>>>(reinterpret_cast<const bf*>(dout), ldo, 0, reinterpret_cast<bf*>(dot), M);
     attn_tc_transpose_kernel<<<gk, block, 0, st>>>(reinterpret_cast<const bf*>(qkv), ld, Hq * HD,
-                                                   reinterpret_cast<bf*>(kt), M, Hkv * HD);
+                                                   reinterpret_cast<bf*>(kt), M);
   }
   CUtensorMap tmQKV128, tmQKV64, tmDO128, tmDO64, tmQt, tmDOt, tmKt;
   int e;
