@@ -149,6 +149,14 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
 // column `col0`.  Rotate-half convention: pair (i, i + hd/2).  sign = +1 forward, -1 inverse.
 // Optional per-head RMSNorm weight (Qwen3 q_norm / k_norm) applied before the rotation
 // is handled by headnorm_* below; here only the rotation.
+// Both forms below turn a pair by the same two roundings per value, written out: left to the compiler, the choice of the
+// product that goes into the fused multiply-add changes with the code around it, and with it some values by one bf16 step.
+__device__ __forceinline__ void rotate_pair(float& x1, float& x2, float c, float s) {
+  const float a = x1, b = x2;
+  x1 = __fmaf_rn(a, c, -__fmul_rn(b, s));
+  x2 = __fmaf_rn(b, c, __fmul_rn(a, s));
+}
+
 // A CTA takes `rows` tokens: the angles of a token are the same for all heads, so their sines and cosines are computed once
 // and read from shared memory, and two units of a thread have their loads in flight together.  16 384 tokens, 32 heads of
 // 128: 107 -> 93 us; the bytes take 42, what is left is the wait for a token's angles before its loads go out.
@@ -184,9 +192,7 @@ rope_kernel(__nv_bfloat16* buf, const int* __restrict__ pos, int M, int ld, int 
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float2 t = x.cs[j];
-      const float x1 = x.a[j], x2 = x.b[j];
-      x.a[j] = x1 * t.x - x2 * t.y;
-      x.b[j] = x2 * t.x + x1 * t.y;
+      rotate_pair(x.a[j], x.b[j], t.x, t.y);
     }
     store8(x.p, x.a);
     store8(x.p + half, x.b);
@@ -226,9 +232,7 @@ __global__ void rope_table_kernel(__nv_bfloat16* __restrict__ buf, const int* __
       sincosf(fp * __ldg(inv_freq + vv * 8 + j), &s, &c);
       s *= sign * mscale;
       c *= mscale;
-      const float x1 = a[j], x2 = b[j];
-      a[j] = x1 * c - x2 * s;
-      b[j] = x2 * c + x1 * s;
+      rotate_pair(a[j], b[j], c, s);
     }
     store8(p, a);
     store8(p + half, b);
