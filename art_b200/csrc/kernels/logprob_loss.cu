@@ -270,12 +270,22 @@ struct EpiSample {
 // Merge sampling partials (over vocabulary splits and, for tensor-parallel heads, over ranks'
 // partial buffers laid out back to back): token id and log-prob per row.
 // One warp per row: a thread per row walked 200 to 300 partials one after another, 20 to 45 us.
+// Of equal scores the lowest token wins, as in sample_restricted.cu and whatever the number of rows: a span's two partials
+// hold the left and the right halves of its tiles, so the order of the partials is not the order of the tokens, and it
+// changes with the tile width.
 __global__ void sample_merge_kernel(const float* __restrict__ partials, int parts, int M, int* __restrict__ token,
                                     float* __restrict__ logprob) {
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (row >= M) return;
   float mx = -INFINITY, sum = 0.f, best = -INFINITY, bx = 0.f;
-  int bi = -1, bs = 0x7fffffff;
+  int bi = -1;
+  auto take = [&](float score, int id, float x) {      // no token (-1) is behind every token
+    if (score > best || (score == best && static_cast<unsigned>(id) < static_cast<unsigned>(bi))) {
+      best = score;
+      bi = id;
+      bx = x;
+    }
+  };
   for (int s = lane; s < parts; s += 32) {
     const float4* p = reinterpret_cast<const float4*>(partials + (static_cast<size_t>(s) * M + row) * 8);
     const float4 a = p[0];
@@ -283,27 +293,17 @@ __global__ void sample_merge_kernel(const float* __restrict__ partials, int part
     const float n = fmaxf(mx, a.x);
     if (n != -INFINITY) sum = sum * __expf(mx - n) + a.y * __expf(a.x - n);
     mx = n;
-    if (a.z > best) {
-      best = a.z;
-      bi = __float_as_int(a.w);
-      bx = x;
-      bs = s;
-    }
+    take(a.z, __float_as_int(a.w), x);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float m2 = __shfl_xor_sync(0xffffffffu, mx, o), s2 = __shfl_xor_sync(0xffffffffu, sum, o);
     const float b2 = __shfl_xor_sync(0xffffffffu, best, o), x2 = __shfl_xor_sync(0xffffffffu, bx, o);
-    const int i2 = __shfl_xor_sync(0xffffffffu, bi, o), p2 = __shfl_xor_sync(0xffffffffu, bs, o);
+    const int i2 = __shfl_xor_sync(0xffffffffu, bi, o);
     const float n = fmaxf(mx, m2);
     if (n != -INFINITY) sum = sum * __expf(mx - n) + s2 * __expf(m2 - n);
     mx = n;
-    if (b2 > best || (b2 == best && p2 < bs)) {      // ties: the first partial, as in one pass
-      best = b2;
-      bi = i2;
-      bx = x2;
-      bs = p2;
-    }
+    take(b2, i2, x2);
   }
   if (lane == 0) {
     token[row] = bi;
