@@ -837,9 +837,9 @@ class NativeRunner(DeviceRunner):
         for i, s in enumerate(seqs):
             nc, n = s.num_cached, len(s.tokens) if s.upto is None else min(s.upto, len(s.tokens))
             new, t = max(0, n - nc), np.arange(max(n, nc))
-            where = np.full(len(t), -1)
-            if write_kv or nc:
-                where = np.asarray(s.blocks)[t // bs] * bs + t % bs
+            where, in_cache = np.full(len(t), -1), t if write_kv else t[:nc]
+            if len(in_cache):
+                where[:len(in_cache)] = np.asarray(s.blocks)[in_cache // bs] * bs + in_cache % bs
             tok.append(np.asarray(s.tokens[nc:n], dtype=np.int64))
             pos.append(t[nc:])
             slot.append(where[nc:] if write_kv else np.full(new, -1))
@@ -872,9 +872,12 @@ class NativeRunner(DeviceRunner):
         run = M > 0 and not cached or len(seqs) == 1        # the new tokens' rows are neighbours
         x = ew.gather_rows(self.embed, t_tok)
 
-        def attend(li):
-            """Attention of the new tokens, whose queries are in ``buf``; keys and values as the cache holds them."""
+        def attend(li, fresh=None):
+            """Attention of the new tokens, keys and values as the cache holds them.  ``fresh``: the new tokens' queries, and
+            their keys and values where the cache does not hold them; None: their queries are in ``buf``."""
             paged.kv_rows(self.kv.k[li], self.kv.v[li], t_held, buf, cfg.q_size, cfg.q_size + cfg.kv_size)
+            if fresh is not None:
+                buf[:, :fresh.shape[1]].index_copy_(0, t_rows, fresh)
             return new_rows(attn_ops.forward(buf, Hq, Hkv, hd, plan, need_grad=False)[0])
 
         def new_rows(o):
@@ -897,8 +900,7 @@ class NativeRunner(DeviceRunner):
             qkv = self._qkv(L, x, t_pos, t_ad, any_lora, out=buf[:M] if place else None)
             paged.kv_write(qkv, cfg.q_size, cfg.q_size + cfg.kv_size, t_slot, self.kv.k[li], self.kv.v[li])
             if cached:
-                buf[:, :cfg.q_size].index_copy_(0, t_rows, qkv[:, :cfg.q_size])
-                o = attend(li)
+                o = attend(li, qkv[:, :cfg.q_size if write_kv else buf.shape[1]])
             else:
                 if not place:
                     buf[:M].copy_(qkv[:, :buf.shape[1]])
