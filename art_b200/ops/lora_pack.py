@@ -48,10 +48,16 @@ class LoraTable:
             for m in lin.members:
                 tensors = (m.a_view, m.b_view, m.ga_view, m.gb_view, lin.A_cat, lin.A_catT, lin.B_cat, lin.B_catT, lin.dA_acc, lin.dB_acc, m.rows)
                 assert all(t.is_contiguous() for t in tensors)
-                n = m.rows.numel()
+                n, r, c0 = m.rows.numel(), self.r, m.slot * self.r
+                # the kernel takes these sizes on trust
+                if c0 + r > lin.kpad:
+                    raise ValueError(f"{m.module}: columns {c0} to {c0 + r} of low-rank operands with {lin.kpad}; adapt the modules "
+                                     "before it as well, or use a lower rank")
+                if lin.r != r or any(t.shape != (r, K) for t in (m.a_view, m.ga_view)) or any(t.shape != (n, r) for t in (m.b_view, m.gb_view)):
+                    raise ValueError(f"{m.module}: factors {tuple(m.a_view.shape)} and {tuple(m.b_view.shape)}, ({r}, {K}) and ({n}, {r}) expected")
                 tiles = (K + TILE - 1) // TILE + (n + TILE - 1) // TILE
                 blocks += [(len(items), t) for t in range(tiles)]
-                items.append(tuple(t.data_ptr() for t in tensors) + (K, n, N, lin.kpad, m.slot * lin.r, 0))
+                items.append(tuple(t.data_ptr() for t in tensors) + (K, n, N, lin.kpad, c0, 0))
         self.items = torch.from_numpy(np.array(items, dtype=_ITEM).view(np.uint8).copy()).to(dev)
         self.blocks = torch.from_numpy(np.array(blocks, dtype=np.int32)).to(dev)
         self.n_blocks = len(blocks)
