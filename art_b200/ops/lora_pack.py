@@ -28,7 +28,8 @@ def _f():
 
 class LoraTable:
     """The members of ``linears`` (``models.native.LoraLinear``) as one table on the device.  Holds the linears, and with them
-    every buffer that the table points to, and gives their gradient accumulators one allocation, cleared by one call."""
+    every buffer that the table points to, and gives their gradient accumulators one allocation, cleared by one call.  Linears
+    that are not on a GPU keep their own copies."""
 
     def __init__(self, linears: list):
         self.linears = [lin for lin in linears if lin.active]
@@ -58,21 +59,28 @@ class LoraTable:
                 tiles = (K + TILE - 1) // TILE + (n + TILE - 1) // TILE
                 blocks += [(len(items), t) for t in range(tiles)]
                 items.append(tuple(t.data_ptr() for t in tensors) + (K, n, N, lin.kpad, c0, 0))
+        if dev.type != "cuda":
+            return
         self.items = torch.from_numpy(np.array(items, dtype=_ITEM).view(np.uint8).copy()).to(dev)
         self.blocks = torch.from_numpy(np.array(blocks, dtype=np.int32)).to(dev)
         self.n_blocks = len(blocks)
 
     def _run(self, export: int) -> None:
-        if self.n_blocks:
-            rc = _f()(_lib.ptr(self.items), _lib.ptr(self.blocks), self.n_blocks, self.r, self.scale, export, _lib.stream_ptr())
-            _lib.check_rc(rc, "lora_pack")
+        rc = _f()(_lib.ptr(self.items), _lib.ptr(self.blocks), self.n_blocks, self.r, self.scale, export, _lib.stream_ptr())
+        _lib.check_rc(rc, "lora_pack")
 
     def refresh(self) -> None:
-        self._run(0)
+        if self.n_blocks:
+            return self._run(0)
+        for lin in self.linears:
+            lin.refresh()
 
     def export_grads(self) -> None:
-        self._run(1)
+        if self.n_blocks:
+            return self._run(1)
+        for lin in self.linears:
+            lin.export_grads()
 
     def zero_grad(self) -> None:
-        if self.n_blocks:
+        if self.linears:
             self.acc.zero_()
