@@ -646,11 +646,14 @@ static int even_grid(int hd, int Hkv) {
   return (shares < 1 ? 1 : shares) * Hkv;
 }
 
-// Bytes of workspace for artb_paged_decode_even: counters [num_seqs * Hkv] (zero before the first call, zero again after
-// each), then two partial results per CTA.
+static int even_part_bytes(int Hq, int Hkv, int hd) { return even_grid(hd, Hkv) * 2 * pa_slot_floats(Hq / Hkv, hd) * 4; }
+
+// Bytes of workspace for artb_paged_decode_even: two partial results per CTA, then counters [num_seqs * Hkv] (zero before the
+// first call, zero again after each).  The counters lie behind what does not depend on the batch, so that a call with fewer
+// sequences leaves those of a larger one as they are.
 ARTB_EXPORT int artb_paged_decode_even_bytes(int num_seqs, int Hq, int Hkv, int hd) {
   if (num_seqs <= 0 || Hkv <= 0 || Hq % Hkv) return 0;
-  return ((num_seqs * Hkv + 3) / 4) * 16 + even_grid(hd, Hkv) * 2 * pa_slot_floats(Hq / Hkv, hd) * 4;
+  return even_part_bytes(Hq, Hkv, hd) + ((num_seqs * Hkv + 3) / 4) * 16;
 }
 
 // The same result with the keys of all sequences in even shares over the chip.  One call at a time may use a workspace.
@@ -665,8 +668,8 @@ ARTB_EXPORT int artb_paged_decode_even(const void* q, int ldq, const void* k_cac
   int dev_ = 0;
   if (cudaGetDevice(&dev_) != cudaSuccess || dev_ < 0 || dev_ >= 64) return ERR_BAD_SHAPE;
   const float scale_log2 = 1.4426950408889634f / sqrtf((float)hd);
-  int* count = static_cast<int*>(ws);
-  float* part = reinterpret_cast<float*>(static_cast<char*>(ws) + ((static_cast<long>(num_seqs) * Hkv + 3) / 4) * 16);
+  float* part = static_cast<float*>(ws);
+  int* count = reinterpret_cast<int*>(static_cast<char*>(ws) + even_part_bytes(Hq, Hkv, hd));
 #define ARTB_PE(HD_)                                                                                                     \
   {                                                                                                                      \
     static bool cfgd[64] = {false};   /* the attribute is per device */                                                  \

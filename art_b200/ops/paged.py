@@ -125,7 +125,7 @@ def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
 
 
 def even_decode_workspace(n: int, Hq: int, Hkv: int, hd: int, device) -> torch.Tensor:
-    """Workspace of :func:`paged_decode_even` for ``n`` sequences; one call at a time may use it."""
+    """Workspace of :func:`paged_decode_even` for up to ``n`` sequences; one call at a time may use it."""
     return torch.zeros(_f("artb_paged_decode_even_bytes")(n, Hq, Hkv, hd), dtype=torch.uint8, device=device)
 
 
