@@ -66,8 +66,10 @@ inline int make_tmap_bf16_2d(CUtensorMap* out, const void* ptr, uint64_t rows, u
 // 2: the second operand of every product launched from now on (a projection's weights, adapter slots included) was
 // written by nothing that could still run, so the product's first weight tiles are requested before the wait.  A decode
 // step alternates products, which stream weights, with short kernels, which leave the memory idle.
+//
+// A thread's own: what holds for the launches of one thread's decode step says nothing of another's products.
 inline int& pdl_switch() {
-  static int on = 0;
+  static thread_local int on = 0;
   return on;
 }
 inline int weights_early() { return pdl_switch() == 2; }

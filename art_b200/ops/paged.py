@@ -56,8 +56,8 @@ def kv_write(qkv: torch.Tensor, k_col: int, v_col: int, slot: torch.Tensor, k_ca
 
 
 def set_pdl(on: bool | int) -> int:
-    """Programmatic dependent launch for the decode-step kernels launched from now on (returns the previous setting):
-    each may start its prologue while its predecessor in the stream drains, and waits on the device before touching
+    """Programmatic dependent launch for the decode-step kernels that this thread launches from now on (returns the previous
+    setting): each may start its prologue while its predecessor in the stream drains, and waits on the device before touching
     global memory.  ``2``: products may also request their second operand (weights that no kernel in flight writes) before
     the wait."""
     return _f("artb_set_pdl")(int(on))
