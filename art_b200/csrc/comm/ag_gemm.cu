@@ -38,6 +38,7 @@ static int launch_ag(const CUtensorMap& tA, const CUtensorMap& tB, const CUtenso
   int cap = sm_count();
   if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
   if (grid > cap) grid = cap;
+  product_overlaps(1);
   kern<<<grid, gemm_pipe_threads<EpiStore<BN>>() + AgComm::THREADS, L::TOTAL, stream>>>(tA, tB, tA2, tB2, kb_main, kb_extra, sched, epi,
                                                                    status, comm);
   return static_cast<int>(cudaGetLastError());
@@ -62,6 +63,7 @@ static int launch_ag_pair(const CUtensorMap& tA, const CUtensorMap& tB, const CU
   int cap = sm_count() / 2;
   if (max_ctas > 0 && max_ctas / 2 < cap) cap = max_ctas / 2 > 0 ? max_ctas / 2 : 1;
   if (clusters > cap) clusters = cap;
+  product_overlaps(2);
   kern<<<2 * clusters, gemm_pipe_threads<EpiStore<256>>() + AgComm::THREADS, L::TOTAL, stream>>>(tA, tB, tA2, tB2, kb_main, kb_extra, sched,
                                                                           epi, status, comm);
   return static_cast<int>(cudaGetLastError());

@@ -125,7 +125,7 @@ struct NoComm {
 };
 
 // Schedules with a member `early` set: B (and B2) are weights that no kernel still running writes, and the loads of the
-// first tile's first stages are issued before the wait for the previous kernel (see pdl_switch in host_utils.h).
+// first tile's first stages are issued before the wait for the previous kernel (see pdl_state in host_utils.h).
 template <class S>
 __device__ __forceinline__ auto sched_early(const S& s, int) -> decltype(s.early) {
   return s.early;

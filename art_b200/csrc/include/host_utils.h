@@ -68,15 +68,32 @@ inline int make_tmap_bf16_2d(CUtensorMap* out, const void* ptr, uint64_t rows, u
 // step alternates products, which stream weights, with short kernels, which leave the memory idle.
 //
 // A thread's own: what holds for the launches of one thread's decode step says nothing of another's products.
-inline int& pdl_switch() {
-  static thread_local int on = 0;
-  return on;
+struct PdlState {
+  int mode = 0;
+  int ctas = 0;      // CTAs per tile of the thread's last product, 0: none since the switch was set
+};
+inline PdlState& pdl_state() {
+  static thread_local PdlState s;
+  return s;
 }
-inline int weights_early() { return pdl_switch() == 2; }
+inline int weights_early() { return pdl_state().mode == 2; }
+
+// Products on single CTAs and on CTA pairs allocate tensor memory in two ways, and decoding has hung where both could be in
+// flight on an SM (the exact interaction was not established).  Kernels release their successor before their own wait, so
+// several launches may be in flight at a time; a product therefore overlaps the launches before it only while they hold
+// products of its own kind.  One of the other kind keeps full stream order: it starts when everything before it has ended,
+// and what overlaps it later comes behind it.  Within a kind no allocation waits for a later kernel, because a kernel is
+// admitted when all CTAs of the one before it have theirs.  Every launch of a product says so here, with or without overlap.
+inline bool product_overlaps(int ctas) {
+  PdlState& s = pdl_state();
+  const bool same = s.ctas == ctas;
+  s.ctas = ctas;
+  return s.mode != 0 && same;
+}
 
 template <class... KArgs, class... Args>
-inline cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                 Args&&... args) {
+inline cudaError_t launch_ordered(bool overlap, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                  Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -86,8 +103,20 @@ inline cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, 
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_switch() ? 1 : 0;
+  cfg.numAttrs = overlap ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
+// kernels without tensor memory
+template <class... KArgs, class... Args>
+inline cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  return launch_ordered(pdl_state().mode != 0, kern, grid, block, smem, stream, static_cast<Args&&>(args)...);
+}
+
+// products with tiles of CTAS CTAs
+template <int CTAS, class... KArgs, class... Args>
+inline cudaError_t launch_product(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  return launch_ordered(product_overlaps(CTAS), kern, grid, block, smem, stream, static_cast<Args&&>(args)...);
 }
 
 inline int sm_count() {

@@ -360,10 +360,13 @@ ARTB_EXPORT int artb_decode_finalize_qkv(float* ws, int ldw, int M, int Hq, int 
   return M <= sm_count() ? go(decode_finalize_qkv_kernel<512>, 512) : go(decode_finalize_qkv_kernel<256>, 256);
 }
 
-// Programmatic dependent launch for the kernels of the decode step (see pdl_switch in host_utils.h); returns the
+// Programmatic dependent launch for the kernels of the decode step (see pdl_state in host_utils.h); returns the
 // previous setting.  The engine turns it on around its decode body and off again afterwards.  2: weights may be read early.
 ARTB_EXPORT int artb_set_pdl(int on) {
-  const int prev = pdl_switch();
-  pdl_switch() = on == 2 ? 2 : on != 0;
+  const int prev = pdl_state().mode;
+  pdl_state() = PdlState{on == 2 ? 2 : on != 0, 0};
   return prev;
 }
+
+// What the launchers ask for each product (1: tiles of one CTA, 2: of CTA pairs): whether it may overlap the launches before it.
+ARTB_EXPORT int artb_product_overlaps(int ctas) { return product_overlaps(ctas); }

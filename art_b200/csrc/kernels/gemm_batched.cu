@@ -60,7 +60,7 @@ static int launch_batched(const CUtensorMap& tA, const CUtensorMap& tB, int kb, 
   }
   int grid = sched.batch * sched.m_tiles * sched.n_tiles;
   if (grid > sm_count()) grid = sm_count();
-  return static_cast<int>(launch_kernel(kern, dim3(grid), dim3(GEMM_THREADS), L::TOTAL, stream, tA, tB, tA, tB, kb, 0, sched, epi,
+  return static_cast<int>(launch_product<1>(kern, dim3(grid), dim3(GEMM_THREADS), L::TOTAL, stream, tA, tB, tA, tB, kb, 0, sched, epi,
                                         status, NoComm{}));
 }
 

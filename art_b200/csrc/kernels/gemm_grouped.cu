@@ -33,6 +33,7 @@ static int launch_grouped(const CUtensorMap& tA, const CUtensorMap& tB, const CU
   }
   int grid = sched.m_tiles * sched.n_tiles;
   if (grid > sm_count()) grid = sm_count();
+  product_overlaps(1);
   kern<<<grid, GEMM_THREADS, L::TOTAL, stream>>>(tA, tB, tA2, tB2, kb_main, kb_extra, sched, epi, status, NoComm{});
   return static_cast<int>(cudaGetLastError());
 }

@@ -38,7 +38,7 @@ static int launch_splitk(const CUtensorMap& tA, const CUtensorMap& tB, int kb_ma
   int grid = sched.m_tiles * sched.n_tiles * splits;
   if (grid > sm_count()) grid = sm_count();
   EpiAtomic<BN> epi{ws, ldw, M, N};
-  return static_cast<int>(launch_kernel(kern, dim3(grid), dim3(GEMM_THREADS), L::TOTAL, stream, tA, tB, tA, tB, kb_main, 0,
+  return static_cast<int>(launch_product<1>(kern, dim3(grid), dim3(GEMM_THREADS), L::TOTAL, stream, tA, tB, tA, tB, kb_main, 0,
                                         sched, epi, status, NoComm{}));
 }
 

@@ -469,7 +469,7 @@ static int launch_lp(const void* H, int ldh, const void* W, int ldw, int M, int 
     sched.m_tiles = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM);      // pair tiles of 256 rows
     int clusters = sched.m_tiles * splits;
     if (clusters > sm_count() / 2) clusters = sm_count() / 2;
-    return static_cast<int>(launch_kernel(kern, dim3(2 * clusters), dim3(gemm_pipe_threads<Epi>()), L::TOTAL, stream, tA, tB,
+    return static_cast<int>(launch_product<2>(kern, dim3(2 * clusters), dim3(gemm_pipe_threads<Epi>()), L::TOTAL, stream, tA, tB,
                                           tA, tB, kb, 0, sched, epi, status, NoComm{}));
   }
   using L = GemmSmemLayout<LP_BN, LP_STAGES>;
@@ -484,7 +484,7 @@ static int launch_lp(const void* H, int ldh, const void* W, int ldw, int M, int 
   sched.m_tiles = (M + GEMM_BM - 1) / GEMM_BM;
   int grid = sched.m_tiles * splits;
   if (grid > sm_count()) grid = sm_count();
-  return static_cast<int>(launch_kernel(kern, dim3(grid), dim3(gemm_pipe_threads<Epi>()), L::TOTAL, stream, tA, tB, tA, tB, kb,
+  return static_cast<int>(launch_product<1>(kern, dim3(grid), dim3(gemm_pipe_threads<Epi>()), L::TOTAL, stream, tA, tB, tA, tB, kb,
                                         0, sched, epi, status, NoComm{}));
 }
 
@@ -639,7 +639,7 @@ static int launch_sample(const void* H, int ldh, const void* W, int ldw, const S
     configured[dev & 63] = true;
   }
   const SchedVocabSpan sched{p.m_tiles, p.n_tiles, p.splits, weights_early()};
-  return static_cast<int>(launch_kernel(kern, dim3(p.m_tiles * p.splits), dim3(gemm_pipe_threads<EpiSample<BN>>()), L::TOTAL,
+  return static_cast<int>(launch_product<1>(kern, dim3(p.m_tiles * p.splits), dim3(gemm_pipe_threads<EpiSample<BN>>()), L::TOTAL,
                                         stream, tA, tB, tA, tB, (K + GEMM_BK - 1) / GEMM_BK, 0, sched, epi, status, NoComm{}));
 }
 
