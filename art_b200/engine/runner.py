@@ -895,6 +895,7 @@ class NativeRunner(DeviceRunner):
                 nxt = self.layers[li + 1]["ln1"] if li + 1 < len(self.layers) else None
                 x, h = self._layer_fused(li, L, x, h, nxt, t_pos, t_slot, t_ad, any_lora, q, attend_q)
             return x, row_ranges
+        whole = not cached and S_att == M       # the projection is the buffer already
         place = not cached and M > 512          # the projection's rows are the buffer's first
         for li, L in enumerate(self.layers):
             qkv = self._qkv(L, x, t_pos, t_ad, any_lora, out=buf[:M] if place else None)
@@ -902,9 +903,9 @@ class NativeRunner(DeviceRunner):
             if cached:
                 o = attend(li, qkv[:, :cfg.q_size if write_kv else buf.shape[1]])
             else:
-                if not place:
+                if not (place or whole):
                     buf[:M].copy_(qkv[:, :buf.shape[1]])
-                o = new_rows(attn_ops.forward(buf, Hq, Hkv, hd, plan, need_grad=False)[0])
+                o = new_rows(attn_ops.forward(qkv if whole else buf, Hq, Hkv, hd, plan, need_grad=False)[0])
             x2 = self._reduce(L["o"](o, t_ad, any_lora, residual=self._res(x)))
             x = self._mlp(L, x2, t_ad, any_lora)
         return x, row_ranges
