@@ -35,6 +35,7 @@ from ..ops import attention as attn_ops
 from ..ops import elementwise as ew
 from ..ops import wgrad
 from ..ops.gemm import gemm_tn, skinny_gemm
+from ..ops.logprob_loss import kept_rows
 from ..ops.lora_pack import LoraTable
 from .config import ModelConfig
 from .weights import LoraConfig, lora_key
@@ -196,11 +197,13 @@ def activation_bytes_per_token(cfg: ModelConfig, mode: str = "none") -> int:
 
 
 def pick_recompute(cfg: ModelConfig, tokens: int, num_layers: int, free_bytes: int) -> str:
-    """The cheapest mode whose saved activations (plus the working set of one layer's backward pass and the LM-head
-    buffers) fit into ``free_bytes``."""
+    """The cheapest mode whose saved activations (plus the working set of one layer's backward pass) fit into ``free_bytes``
+    with a margin, which also has room for the logits that the LM head keeps (at worst all tokens are trainable)."""
+    logits = 4 * kept_rows(tokens) * cfg.vocab_size
     work = tokens * (4 * activation_bytes_per_token(cfg, "none") + 16 * cfg.hidden_size)
     for mode in RECOMPUTE_MODES:
-        if tokens * num_layers * activation_bytes_per_token(cfg, mode) + work <= 0.85 * free_bytes:
+        held = tokens * num_layers * activation_bytes_per_token(cfg, mode) + work
+        if held <= 0.85 * free_bytes and held + logits <= 0.95 * free_bytes:
             return mode
     return "full"
 

@@ -100,6 +100,11 @@ def backward(hidden, lm_head, lm_head_t, target, lse, coef, dlogits_buf: torch.T
 LOGIT_ROWS = 2048     # at most this many rows' logits are alive at once, or half of the batch's (see forward_backward)
 
 
+def kept_rows(M: int) -> int:
+    """How many of ``M`` rows :func:`forward_backward` keeps the logits of at a time."""
+    return min(M, max(LOGIT_ROWS, ((M + 1) // 2 + 255) // 256 * 256))
+
+
 def forward_backward(hidden, lm_head, lm_head_t, target, old_lp, adv, tok_w, ref_lp=None, eps_lo=0.2, eps_hi=0.2, beta=0.0,
                      accum=None) -> tuple[LogprobResult, torch.Tensor]:
     """Loss terms of the rows of ``hidden`` and dLoss/dhidden [M,K] bf16, the logits computed once.
@@ -109,9 +114,9 @@ def forward_backward(hidden, lm_head, lm_head_t, target, old_lp, adv, tok_w, ref
     """
     M, K = hidden.shape
     V, ldl = lm_head.shape[0], lm_head_t.shape[1]
-    piece = max(LOGIT_ROWS, ((M + 1) // 2 + 255) // 256 * 256)
+    piece = kept_rows(M)
     dh = torch.empty((M, K), dtype=torch.bfloat16, device=hidden.device)
-    buf = torch.empty((min(piece, M), ldl), dtype=torch.float32, device=hidden.device)
+    buf = torch.empty((piece, ldl), dtype=torch.float32, device=hidden.device)
     parts = []
     for m0 in range(0, M, piece):
         s = slice(m0, min(M, m0 + piece))
