@@ -725,8 +725,8 @@ class HybridRunner(DeviceRunner):
         # of whole 256 rows, which keep full stream order between kernels.
         return nb % 256 != 0
 
-    def _attn_splits(self, nb: int, max_ctx: int) -> int:
-        """Stands for how far the batch's tokens reach back (a power of two): the attention layers plan their splits by it.
+    def _reach(self, max_ctx: int) -> int:
+        """How far the batch's tokens reach back (a power of two): the attention layers plan their splits by it.
         Contexts beyond every window and chunk change nothing, so that they share one captured graph."""
         windows = [s.window or s.chunk for L in self.cfg.layers for s in L.mixers() if s.type in ("latent_attention", "attention")]
         if not windows:
@@ -734,19 +734,16 @@ class HybridRunner(DeviceRunner):
         bound = max_ctx if any(w <= 0 for w in windows) else min(max_ctx, max(windows))
         return 1 << max(0, bound - 1).bit_length()
 
-    def _attn_workspace(self, nb: int, splits: int) -> None:
-        return None
-
     def drop_graphs(self) -> None:
         super().drop_graphs()
         self._buf.clear()         # workspaces of an interrupted step may hold partial sums
 
-    def _decode_steps(self, st, n_steps: int, any_lora: bool, splits: int, ws, restricted: bool, procs) -> None:
+    def _decode_steps(self, st, n_steps: int, any_lora: bool, reach: int, restricted: bool, procs) -> None:
         from ..ops import paged
 
         nb = st["tokens"].shape[0]
         b = Ragged(nb, nb, st["tokens"], st["pos"], st["slot"], st["row_seq"], st["cu_q"], st["ctx"], st["state_slot"], st["bt"], True,
-                   n_abs=nb, reach=splits)
+                   n_abs=nb, reach=reach)
         for k in range(n_steps):
             _, hidden = self._forward(b, want_hidden=True)
             t, lp = self._sample(hidden, st["inv_t"], st["seeds"][k], restricted, st["top_k"], st["top_p"], st["min_p"], procs=procs)

@@ -356,7 +356,7 @@ class DeviceRunner:
     ``_hidden_rows(x, rows)``                 final norm of chosen rows
     ``_decode_steps(st, ...)``                n decode steps on the staged buffers
     ``_decode_buffers / _stage_sequences``    further per-sequence buffers of a decode batch and how they are filled
-    ``_attn_splits / _attn_workspace``        split-KV plan of the decode attention
+    ``_reach(max_ctx)``                       what the plans of a decode batch, and with them its captured graph, depend on
     """
 
     tp, tp_group, tp_rank = 1, None, 0
@@ -370,6 +370,9 @@ class DeviceRunner:
 
     def _stage_sequences(self, st, seqs, nb: int) -> None:
         pass
+
+    def _reach(self, max_ctx: int) -> int:
+        return 0
 
     def close(self) -> None:
         """Drop the captured decode graphs and their buffers.  A tensor-parallel runner must be closed before its
@@ -489,7 +492,7 @@ class DeviceRunner:
     # The multi-step decode runs on persistent device buffers (one set per batch-size bucket) so that
     # the whole run of n_steps x (all layers + sampler + state advance) can be captured in a CUDA
     # graph and replayed: a decode step is ~500 small launches, which the host cannot issue as fast
-    # as the GPU retires them.  The first use of a (bucket, n_steps, lora, splits, table width) key
+    # as the GPU retires them.  The first use of a (bucket, n_steps, lora, reach, table width) key
     # runs eagerly, the second captures, later ones replay.
     BUCKETS = (8, 16, 32, 64, 128, 256, 512, 1024)
 
@@ -519,12 +522,12 @@ class DeviceRunner:
     def _overlap(self, nb: int) -> bool:
         return self.overlap_launches
 
-    def _decode_body(self, st, n_steps: int, any_lora: bool, splits: int, ws, restricted: bool = False, procs=None):
+    def _decode_body(self, st, n_steps: int, any_lora: bool, reach: int, restricted: bool = False, procs=None):
         from ..ops import paged
 
         prev_pdl = paged.set_pdl(2 if self._overlap(st["tokens"].shape[0]) and os.environ.get("ARTB_PDL", "1") != "0" else 0)
         try:
-            self._decode_steps(st, n_steps, any_lora, splits, ws, restricted, procs)
+            self._decode_steps(st, n_steps, any_lora, reach, restricted, procs)
         finally:
             paged.set_pdl(prev_pdl)
 
@@ -590,17 +593,12 @@ class DeviceRunner:
             st["top_p"].copy_(torch.tensor([s.top_p for s in seqs] + [1.0] * pad, dtype=torch.float32), non_blocking=True)
             st["min_p"].copy_(torch.tensor([s.min_p for s in seqs] + [0.0] * pad, dtype=torch.float32), non_blocking=True)
         max_ctx = max(lens) + n_steps
-        splits = self._attn_splits(nb, max_ctx)
-        key = (nb, max_blocks, n_steps, any_lora, splits, restricted, self._moe_mixed)
-        ws = None
-        if splits > 1:
-            ws = st.get(("ws", splits))
-            if ws is None:
-                ws = st[("ws", splits)] = self._attn_workspace(nb, splits)
+        reach = self._reach(max_ctx)
+        key = (nb, max_blocks, n_steps, any_lora, reach, restricted, self._moe_mixed)
         graph = self._dgraphs.get(key) if procs is None else None
         self.last_top_logprobs = None
         if procs is not None:
-            self._decode_body(st, 1, any_lora, splits, ws, True, procs=procs)
+            self._decode_body(st, 1, any_lora, reach, True, procs=procs)
             self.last_top_logprobs = [self._step_top] if self._step_top is not None else None
         elif graph is not None:
             graph.replay()
@@ -608,12 +606,12 @@ class DeviceRunner:
             torch.cuda.synchronize()
             graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(graph):
-                self._decode_body(st, n_steps, any_lora, splits, ws, restricted)
+                self._decode_body(st, n_steps, any_lora, reach, restricted)
             self._dgraphs[key] = graph
             graph.replay()
         else:
             self._dseen.add(key)
-            self._decode_body(st, n_steps, any_lora, splits, ws, restricted)
+            self._decode_body(st, n_steps, any_lora, reach, restricted)
         out_t = st["out_t"][:, :n].tolist()
         out_l = st["out_l"][:, :n].tolist()
         return out_t, out_l
@@ -931,7 +929,7 @@ class NativeRunner(DeviceRunner):
         part, _ = lpl.partials(h, self.lm_head, tgt)
         return lpl.grpo_tokens(part).logprobs.tolist()
 
-    def _decode_steps(self, st, n_steps: int, any_lora: bool, splits: int, ws, restricted: bool, procs) -> None:
+    def _decode_steps(self, st, n_steps: int, any_lora: bool, reach: int, restricted: bool, procs) -> None:
         from ..ops import elementwise as ew
         from ..ops import paged
 
@@ -1021,6 +1019,3 @@ class NativeRunner(DeviceRunner):
         return {"attn_out": torch.zeros((nb, cfg.q_size), dtype=torch.bfloat16, device=self.device),
                 "q": torch.zeros((nb, cfg.q_size), dtype=torch.bfloat16, device=self.device),
                 "attn_ws": paged.even_decode_workspace(nb, cfg.num_heads, cfg.num_kv_heads, cfg.head_dim, self.device)}
-
-    def _attn_splits(self, nb: int, max_ctx: int) -> int:
-        return 1        # the decode attention shares the keys out by itself, on the device
