@@ -695,7 +695,7 @@ attn_tc_dq_kernel(const __grid_constant__ CUtensorMap tmQKV128, const __grid_con
 
 // dk|dv rows = sum over the GS partials (dk scaled), written as bf16 into the k|v columns of dqkv
 __global__ void attn_tc_combine_dkv_kernel(const float* __restrict__ partial, int GS, __nv_bfloat16* __restrict__ dqkv, int ld,
-                                           int kcol0, long M, int kvw /* Hkv * 128 */, float scale) {
+                                           int kcol0, long M, int kvw /* Hkv * HD */, float scale) {
   const int vec = (2 * kvw) >> 2;
   const long total = M * vec;
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < total;

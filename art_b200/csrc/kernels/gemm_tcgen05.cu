@@ -89,7 +89,8 @@ ARTB_EXPORT int artb_gemm_bf16_tn(const void* A, int lda, const void* B, int ldb
   if (bn == 0) bn = artb_pick_bn(M, N, max_ctas > 0 && max_ctas < sm_count() ? max_ctas : sm_count());
   if (bn != 64 && bn != 128 && bn != 160 && bn != 192 && bn != 224 && bn != 256) return ERR_BAD_SHAPE;
 
-  // few rows: stages with as many rows of A as there are, and more of them
+  // few rows: stages with as many rows of A as there are, and more of them (64 and 224 columns keep whole tiles of A: shorter
+  // ones have not been measured there)
   const int ar = bn < 128 || bn == 224 || M > 64 ? GEMM_BM : M > 16 ? 64 : 16;
   CUtensorMap tA, tB, tA2, tB2;
   int e;

@@ -13,7 +13,8 @@
 //     dlogit[t, v] = coef[t] * (onehot(target_t)[v] - exp(logit[t, v] - lse[t]))
 // as bf16; a plain TN GEMM against the resident transposed LM head then gives dH.  A training step lets the forward
 // write its logits in fp32 for a bounded number of rows and turns them into dlogits in place (dlogits_inplace_kernel);
-// a caller that kept no logits recomputes the tiles with the same pipeline (EpiDLogits).
+// a caller that kept no logits recomputes the tiles with the same pipeline (EpiDLogits: the separate forward and backward of
+// ops/logprob_loss.py; no training step takes them).
 // In a vocab-parallel (TP) layout each rank runs this over its vocabulary shard and
 // the 3-float partials are what ranks exchange.
 //

@@ -73,7 +73,8 @@ __global__ void kv_write_kernel(const __nv_bfloat16* __restrict__ qkv, int ld, i
   }
 }
 
-// Gather the first n_tok cached tokens of one sequence into contiguous k | v columns of dst [*, ld].
+// Gather the first n_tok cached tokens of one sequence into contiguous k | v columns of dst [*, ld] (prompt steps take all
+// their sequences' rows at once: kv_rows below).
 __global__ void kv_gather_kernel(const __nv_bfloat16* __restrict__ k_cache, const __nv_bfloat16* __restrict__ v_cache,
                                  const int* __restrict__ block_table, int block_size, int n_tok,
                                  __nv_bfloat16* __restrict__ dst, int ld, int k_col, int v_col, int kv_width,
