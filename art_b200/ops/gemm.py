@@ -7,6 +7,7 @@ PyTorch restatement used by the tests.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 
 import torch
@@ -213,6 +214,7 @@ def splitk_finalize(ws: torch.Tensor, out: torch.Tensor, bias: torch.Tensor | No
     return out
 
 
+@functools.lru_cache(maxsize=4096)      # a first pass over a batch issues a few hundred products a step from the host
 def plan_small_m(M: int, N: int, K: int, sms: int = 148, pair: bool = False) -> tuple[int, int]:
     """(bn, splits) for a weight-streaming GEMM: widest N tile, then split K as far as ONE wave of CTAs allows
     (tiles * splits <= SMs: a second, nearly empty wave would double the time).  ``pair``: 256 x 256 tiles on CTA
@@ -235,6 +237,7 @@ def plan_small_m(M: int, N: int, K: int, sms: int = 148, pair: bool = False) -> 
     return bn, splits
 
 
+@functools.lru_cache(maxsize=4096)
 def stream_bn(M: int, N: int, sms: int = 148) -> int:
     """Tile width of an unsplit weight-streaming GEMM of up to 256 rows: the one whose busiest CTA streams the fewest
     weight rows, the widest where they tie.  22016 x 2048 weights are 86 tiles of 256 or 138 of 160; 24576 x 4096 are 192

@@ -3,6 +3,7 @@ multi-LoRA slot mask, fused LM-head sampler, top-k / top-p sampler, device-side 
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import torch
 
@@ -124,16 +125,21 @@ def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
     return out
 
 
+@functools.lru_cache(maxsize=1024)
+def _even_bytes(n: int, Hq: int, Hkv: int, hd: int, device: int | None) -> int:
+    return _f("artb_paged_decode_even_bytes")(n, Hq, Hkv, hd)
+
+
 def even_decode_workspace(n: int, Hq: int, Hkv: int, hd: int, device) -> torch.Tensor:
     """Workspace of :func:`paged_decode_even` for up to ``n`` sequences; one call at a time may use it."""
-    return torch.zeros(_f("artb_paged_decode_even_bytes")(n, Hq, Hkv, hd), dtype=torch.uint8, device=device)
+    return torch.zeros(_even_bytes(n, Hq, Hkv, hd, torch.device(device).index), dtype=torch.uint8, device=device)
 
 
 def paged_decode_even(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,
                       ctx_len: torch.Tensor, Hq: int, Hkv: int, hd: int, out: torch.Tensor, ws: torch.Tensor) -> torch.Tensor:
     """:func:`paged_decode` with the keys of all sequences in even shares over the chip, whatever their lengths."""
     n = q.shape[0]
-    need = _f("artb_paged_decode_even_bytes")(n, Hq, Hkv, hd)
+    need = _even_bytes(n, Hq, Hkv, hd, q.device.index)
     if ws.numel() * ws.element_size() < need:
         raise ValueError(f"workspace of {ws.numel() * ws.element_size()} bytes, {need} needed")
     _lib.check_rc(_f("artb_paged_decode_even")(_lib.ptr(q), q.stride(0), _lib.ptr(k_cache), _lib.ptr(v_cache),
